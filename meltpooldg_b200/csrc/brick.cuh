@@ -47,6 +47,7 @@ namespace mpdg
     const uint8_t *cmask;  // optional per-DoF Dirichlet flags (device), may be null
     unsigned       acc_lo_z = 0; // the lattice is a z-slab of a larger one: its low z plane already
                                  // holds the previous slab's contributions and is only added into
+    int            bz = 0;       // cell layers per segment of the column-marching apply (march.cuh)
   };
 
   constexpr unsigned SPIN_LIMIT    = 1u << 22; // x 32 ns sleeps: ~0.1-0.2 s

@@ -1148,6 +1148,8 @@ mpdg_op_create(const mpdg_mesh_desc *mesh, const mpdg_op_params *params, mpdg_op
   // at k <= 3, the advection-form kernels of its convection velocity, on their own bricks)
   long long nbrk = std::max((long long)op->nbr[0] * op->nbr[1] * op->nbr[2],
                             (long long)op->nbr32[0] * op->nbr32[1] * op->nbr32[2]);
+  if (op->kind == MPDG_HEAT)
+    nbrk = std::max(nbrk, heat_flags(op->degree, op->m, mesh->dirichlet_mask == nullptr));
   if (op->kind == MPDG_HEAT && op->degree <= 3)
     for (int prec = 0; prec < 2; ++prec)
       {

@@ -308,17 +308,20 @@ namespace mpdg
   {
     static constexpr int N = K + 1, NE = (N + 1) / 2, NO = N / 2;
     const HeatArgs<T, N> &a;
+    // conductivity of the cell (unscaled)
+    __device__ __forceinline__ T
+    load(bool valid, int cx, int cy, int cz) const
+    {
+      if (!a.kcell)
+        return a.kconst;
+      return valid ? a.kcell[(long long)cx + (long long)a.g.m[0] * ((long long)cy + (long long)a.g.m[1] * cz)] : T(0);
+    }
     template <bool DOT>
     __device__ __forceinline__ double
-    apply(T *u, bool valid, int cx, int cy, int cz) const
+    apply(T *u, T k) const
     {
-      T form = T(0);
-      T kc = T(0);
-      if (valid)
-        {
-          const long long c = (long long)cx + (long long)a.g.m[0] * ((long long)cy + (long long)a.g.m[1] * cz);
-          kc                = a.kscale * (a.kcell ? a.kcell[c] : a.kconst);
-        }
+      T       form = T(0);
+      const T kc   = a.kscale * k;
       const T *tb  = fd_table<T>(K);
       const T *we  = tb;
       const T *wo  = tb + NE * NE;
@@ -356,30 +359,38 @@ namespace mpdg
   };
 
 #ifndef MPDG_MARCH_MINB_F64
-#define MPDG_MARCH_MINB_F64 5
+#define MPDG_MARCH_MINB_F64 4
 #endif
 #ifndef MPDG_MARCH_MINB_F32
-#define MPDG_MARCH_MINB_F32 8
+#define MPDG_MARCH_MINB_F32 7
+#endif
+#ifndef MPDG_MARCH_MINB1_F64
+#define MPDG_MARCH_MINB1_F64 10
+#endif
+#ifndef MPDG_MARCH_MINB1_F32
+#define MPDG_MARCH_MINB1_F32 10
 #endif
   // CTAs per SM the register allocation of the column-marching kernel is held to
-  template <typename T>
+  template <int K, typename T>
   struct MarchMinBlocks
   {
-    static constexpr int value = sizeof(T) == 8 ? MPDG_MARCH_MINB_F64 : MPDG_MARCH_MINB_F32;
+    static constexpr int value = K == 1 ? (sizeof(T) == 8 ? MPDG_MARCH_MINB1_F64 : MPDG_MARCH_MINB1_F32)
+                                        : (sizeof(T) == 8 ? MPDG_MARCH_MINB_F64 : MPDG_MARCH_MINB_F32);
   };
 
   template <int K, typename T, OutMode MODE, bool DOT>
-  __global__ void __launch_bounds__(MarchShape<K, T>::NT, MarchMinBlocks<T>::value)
+  __global__ void __launch_bounds__(MARCH_NT, MarchMinBlocks<K, T>::value)
   heat_march_kernel(const __grid_constant__ HeatArgs<T, K + 1> a)
   {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned s_ticket;
-    __shared__ double   s_red[MarchShape<K, T>::NT / 32];
+    __shared__ unsigned                         s_ticket;
+    __shared__ double                           s_red[MARCH_NT / 32];
+    __shared__ __align__(8) unsigned long long  s_bars[2];
     if (a.skip != nullptr && *a.skip != 0)
       return;
     HeatCellOp<K, T> op{a};
     march_body<K, T, MODE, HeatCellOp<K, T>, DOT>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
-                                                  reinterpret_cast<T *>(smem_raw), &s_ticket, a.dot, s_red);
+                                                  reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars, a.dot, s_red);
   }
 
   // ---- k >= 3: pencil-marching apply (pencil.cuh); the x lines are scaled by the diagonal of the
@@ -595,11 +606,12 @@ namespace mpdg
     a.mask_src = h.mask_src;
     a.skip     = h.skip;
     a.dot      = h.dot;
-    const unsigned nbricks = (unsigned)h.grid.nbr[0] * h.grid.nbr[1] * h.grid.nbr[2];
     if constexpr (K <= 2)
       if (h.grid.cmask == nullptr && h.march)
         {
           using ML = MarchLayout<K, T>;
+          a.g.bz = march_plan(a.g.m, MarchShape<K, T>::BZ, 148 * MarchMinBlocks<K, T>::value, &a.g.nbr[2]);
+          const unsigned nbricks = (unsigned)a.g.nbr[0] * a.g.nbr[1] * a.g.nbr[2];
           static std::atomic<unsigned long long> dev_plain{0}, dev_dot{0};
           if constexpr (MODE == OutMode::Set)
             if (h.dot.part != nullptr)
@@ -608,16 +620,17 @@ namespace mpdg
                 cudaError_t e    = ensure_smem(kern, ML::bytes, dev_dot);
                 if (e != cudaSuccess)
                   return e;
-                kern<<<nbricks, ML::S::NT, ML::bytes, stream>>>(a);
+                kern<<<nbricks, MARCH_NT, ML::bytes, stream>>>(a);
                 return cudaGetLastError();
               }
           auto        kern = heat_march_kernel<K, T, MODE, false>;
           cudaError_t e    = ensure_smem(kern, ML::bytes, dev_plain);
           if (e != cudaSuccess)
             return e;
-          kern<<<nbricks, ML::S::NT, ML::bytes, stream>>>(a);
+          kern<<<nbricks, MARCH_NT, ML::bytes, stream>>>(a);
           return cudaGetLastError();
         }
+    const unsigned nbricks = (unsigned)h.grid.nbr[0] * h.grid.nbr[1] * h.grid.nbr[2];
     if constexpr (K >= 3)
       if (h.grid.cmask == nullptr && h.march)
         {
@@ -686,6 +699,28 @@ namespace mpdg
         shape[1] = K == 1 ? HeatBrickShape<1, T>::BY : HeatBrickShape<2, T>::BY;
         shape[2] = K == 1 ? HeatBrickShape<1, T>::BZ : HeatBrickShape<2, T>::BZ;
       }
+  }
+
+  long long
+  heat_flags(int K, const int m[3], bool march)
+  {
+    if (march && K <= 2)
+      return std::max(march_flags(m, K == 1 ? MarchShape<1, double>::BZ : MarchShape<2, double>::BZ),
+                      march_flags(m, K == 1 ? MarchShape<1, float>::BZ : MarchShape<2, float>::BZ));
+    long long most = 1;
+    for (int prec = 0; prec < 2; ++prec)
+      {
+        int sh[3];
+        if (prec == 0)
+          heat_brick_shape<double>(K, sh, march);
+        else
+          heat_brick_shape<float>(K, sh, march);
+        long long nb = 1;
+        for (int d = 0; d < 3; ++d)
+          nb *= (m[d] + sh[d] - 1) / sh[d];
+        most = std::max(most, nb);
+      }
+    return most;
   }
 
   template <int K, typename T>

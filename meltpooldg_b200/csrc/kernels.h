@@ -49,6 +49,8 @@ namespace mpdg
 
   template <typename T>
   void heat_brick_shape(int K, int shape[3], bool march);
+  // init flags (and fused-dot partials) that an apply of this mesh may use, in either precision
+  long long heat_flags(int K, const int m[3], bool march);
 
   // ---- boundary-face terms of the heat operator (faces.cu); face f: bit 2d low / 2d+1 high of dim d
   struct HeatFaceBC

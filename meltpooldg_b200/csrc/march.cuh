@@ -1,236 +1,572 @@
-// Column-marching apply for low degrees (k <= 2): one thread per cell, no shared-memory reduction.
+// Column-marching apply for low degrees: one thread per cell, no shared-memory reduction.
 //
-// A CTA of 4 warps owns a column of 32 x 4 cells (x, y) and marches through a segment of BZ cell
+// A CTA of 4 warps owns a column of 32 x 4 cells (x, y) and marches through a segment of bz cell
 // layers in z.  Lane = cell x-index, warp = cell y-index.  Per layer:
-//   1. the (k+1) lattice planes of the layer are staged into shared memory with cp.async (double
-//      buffered: the next layer is in flight while the current one is computed);
-//   2. each thread applies the cell operator to its cell's (k+1)^3 values in registers;
-//   3. x-neighbours combine their common face with warp shuffles (lane t adds lane t-1's x = k face
-//      into its x = 0 face), y-neighbours through a small shared exchange buffer, z-neighbours by
-//      carrying the z = k face in registers to the next layer of the same thread;
-//   4. each thread then owns the points i, j, l in [0, k) of its cell (plus the column's high faces
-//      for the last lane / warp / layer) and writes them to global memory with coalesced stores.
-// Points on the faces shared with neighbouring columns / segments are combined with global atomics,
-// initialised by their owner through the ticket / flag handshake of brick.cuh.
+//   1. the K new lattice planes of the layer arrive in a ring of 2 K + 1 planes by bulk copies
+//      (cp.async.bulk, one per lattice row, issued by the lanes of warp 0 two layers ahead); the plane
+//      shared with the layer below stays in the ring;
+//   2. each thread applies the cell operator to its cell's (K+1)^3 values in registers;
+//   3. x-neighbours combine their common face with warp shuffles (lane t adds lane t-1's x = K face
+//      into its x = 0 face), y-neighbours through a small shared exchange buffer (two buffers taken in
+//      turn: one barrier per layer), z-neighbours by carrying the z = K face in registers;
+//   4. each thread then owns the points i, j, l in [0, K) of its cell and writes them with coalesced
+//      stores; points on the faces shared with neighbouring columns / segments are combined with global
+//      atomics, initialised by their owner through the ticket / flag handshake of brick.cuh.  The
+//      column's high x face (one lane) and high y face (one warp) add straight from the cell's values,
+//      so neither the exchange nor the carry handles them.
+//
+// Staging.  A lattice row of n points starts at any element, a bulk copy at a 16-byte boundary: the copy
+// starts at the boundary below the row's first point, and the row sits in its slot shifted by the
+// elements in between, (address / sizeof(T)) mod (16 / sizeof(T)), which every reader computes from the
+// row's index.  Granules that would reach outside the vector (its first and last row only) are fetched
+// point by point.  Against per-element copies (cp.async of all K + 1 planes by every thread, with the
+// row and bounds arithmetic of each point) this took the FE_Q(2) FP64 apply from 1439 to about 1000 warp
+// instructions per 32 cells; the kernel is bound by instruction issue and latency, not by bandwidth.
+//
+// Segment length.  bz is chosen per mesh by march_plan (below).
 #pragma once
+
+#include <type_traits>
 
 #include "brick.cuh"
 
 namespace mpdg
 {
-#ifndef MPDG_MARCH_BZ2_F32
-#define MPDG_MARCH_BZ2_F32 16
-#endif
-  // Cell layers per column segment: longer segments amortise the brick handshake and the staging
-  // prologue; for k = 2 in FP64 the 8-layer segment gives more CTAs per wave and wins.
+  constexpr int MARCH_BX = 32, MARCH_BY = 4, MARCH_NT = 128;
+  // segments of any mesh: at most the full-length ones or this many (brick flags, dot partials)
+  constexpr long long MARCH_MIN_FLAGS = 8192;
+
+  // Cell layers of a full-length segment (the handle's brick count, and the bound of the flags on
+  // large meshes).
   template <int K, typename T>
   struct MarchShape
   {
-    static constexpr int BX = 32, BY = 4, NT = 128;
-    static constexpr int BZ = K == 1 ? 16 : (sizeof(T) == 4 ? MPDG_MARCH_BZ2_F32 : 8);
+    static constexpr int BX = MARCH_BX, BY = MARCH_BY, NT = MARCH_NT;
+    static constexpr int BZ = K == 1 ? 16 : (sizeof(T) == 4 ? 16 : 8);
   };
+
+  // Segment length for a mesh: the bz whose CTAs take the least time on the resident slots.  In units of
+  // a layer at full occupancy a CTA costs its layers plus about one (two, where it starts on an idle
+  // slot: handshake and the first planes' latency); the last wave, of which only a part of the slots is
+  // in use, takes 0.57 + 0.43 part of that per layer (FE_Q(2) FP64, 96^3: 5.6 us a layer at 4.9 CTAs
+  // per SM, 4.5 at 2.9, 3.9 at 1.5).  Measured against it, FE_Q(2) FP64: 96^3 67 us at bz = 10 (one
+  // full wave) against 88 at 8 (864 segments on 740 slots) and 81 at 16; 64^3 25 us at 3 against 36 at
+  // 8; 32^3 10 us at 1 against 33 at 8.
+  inline int
+  march_plan(const int m[3], int bz_full, int slots, int *nseg)
+  {
+    const long long cols = (long long)((m[0] + MARCH_BX - 1) / MARCH_BX) * ((m[1] + MARCH_BY - 1) / MARCH_BY);
+    const long long cap  = cols * ((m[2] + bz_full - 1) / bz_full);
+    double          best = 0.0;
+    int             bz   = bz_full;
+    for (int b = 1; b <= 32 && (b <= m[2] || b == 1); ++b)
+      {
+        const long long nb = cols * ((m[2] + b - 1) / b);
+        if (nb > cap && nb > MARCH_MIN_FLAGS)
+          continue;
+        const long long full = nb / slots;
+        const double    part = (double)(nb % slots) / slots;
+        const double    cost = (b + 1.0) * (double)full + (part > 0.0 ? (b + 2.0) * (0.57 + 0.43 * part) : 0.0);
+        if (best == 0.0 || cost < best)
+          {
+            best = cost;
+            bz   = b;
+          }
+      }
+    *nseg = (m[2] + bz - 1) / bz;
+    return bz;
+  }
+
+  // flags / dot partials an operator must hold for the segments of any of its marching applies
+  inline long long
+  march_flags(const int m[3], int bz_full)
+  {
+    const long long cols = (long long)((m[0] + MARCH_BX - 1) / MARCH_BX) * ((m[1] + MARCH_BY - 1) / MARCH_BY);
+    const long long cap  = cols * ((m[2] + bz_full - 1) / bz_full);
+    return cap > MARCH_MIN_FLAGS ? cap : MARCH_MIN_FLAGS;
+  }
 
   template <int K, typename T>
   struct MarchLayout
   {
-    using S                 = MarchShape<K, T>;
-    static constexpr int N  = K + 1;
-    static constexpr int PX = K * S::BX + 1, PY = K * S::BY + 1, NPL = K + 1;
-    static constexpr int LAYER = NPL * PY * PX;           // staged points per layer
-    static constexpr int YX    = S::BY * N * N * 32;      // y-exchange buffer
-    static constexpr size_t bytes = sizeof(T) * (2 * (size_t)LAYER + YX);
-    using BR = Brick<K, S::BX, S::BY, S::BZ, S::NT>;      // geometry / handshake of the column segment
+    static constexpr int N = K + 1, G = 16 / (int)sizeof(T);
+    static constexpr int PX = K * MARCH_BX + 1, PY = K * MARCH_BY + 1, NRING = 2 * K + 1;
+    static constexpr int PITCH = (PX + G - 1 + G - 1) / G * G; // row of a slot: shift + points
+    static constexpr int PLANE = PY * PITCH;
+    static constexpr int YX    = MARCH_BY * N * K * 32;        // y-exchange, one buffer
+    static constexpr size_t bytes = sizeof(T) * (NRING * (size_t)PLANE + 2 * (size_t)YX);
   };
 
-  // Stage layer lz of the column into buf (cp.async; zeros outside the domain and, with mask, on
-  // Dirichlet planes -- decided per row plus two compares per point).
-  template <class LAY, class BR, typename T>
-  __device__ __forceinline__ void
-  march_stage(const BR &br, int lz, const T *src, bool mask, T *buf)
+  // Geometry of one column segment (K points per cell; bz layers)
+  template <int K>
+  struct Column
   {
-    constexpr int K = LAY::N - 1;
-    constexpr int PX = LAY::PX, PY = LAY::PY, NR = LAY::NPL * PY;
+    int      c0[3], g0[3], nv[3];
+    int      lo_sh[3], hi_sh[3], con_lo[3], con_hi[3], any_con;
+    int      sy, sz, layers;
+    unsigned id;
+    __device__ __forceinline__ void
+    set(const GridDesc &g, unsigned t)
+    {
+      id           = t;
+      const int B[3] = {MARCH_BX, MARCH_BY, g.bz};
+      c0[0]        = (int)(t % (unsigned)g.nbr[0]) * MARCH_BX;
+      c0[1]        = (int)((t / (unsigned)g.nbr[0]) % (unsigned)g.nbr[1]) * MARCH_BY;
+      c0[2]        = (int)(t / (unsigned)(g.nbr[0] * g.nbr[1])) * g.bz;
+      any_con      = 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        {
+          g0[d]     = K * c0[d];
+          nv[d]     = min(K * B[d] + 1, g.n[d] - g0[d]);
+          lo_sh[d]  = c0[d] > 0;
+          hi_sh[d]  = c0[d] + B[d] < g.m[d];
+          con_lo[d] = ((g.faces >> (2 * d)) & 1u) && g0[d] == 0;
+          con_hi[d] = ((g.faces >> (2 * d + 1)) & 1u) && g0[d] + nv[d] == g.n[d];
+          any_con |= con_lo[d] | con_hi[d];
+        }
+      sy     = g.n[0];
+      sz     = g.n[0] * g.n[1];
+      layers = min(g.bz, g.m[2] - c0[2]);
+    }
+    __device__ __forceinline__ int
+    index(int px, int py, int pz) const
+    {
+      return (g0[0] + px) + sy * (g0[1] + py) + sz * (g0[2] + pz);
+    }
+    __device__ __forceinline__ bool
+    has_lower_neighbour() const
+    {
+      return lo_sh[0] || lo_sh[1] || lo_sh[2];
+    }
+  };
+
+  // Initialise the face points the segment owns (Set: 0, BPlus: b) and publish the flag: its high faces
+  // and, at the domain's low boundary, its low faces (edge points are visited up to three times with the
+  // same value).  acc_lo_z: the lattice's low z plane holds the previous slab's values and stays.
+  template <int K, typename T, OutMode MODE>
+  __device__ __forceinline__ void
+  column_init_publish(const Column<K> &br, const SyncDesc &s, T *dst, const T *bvec, unsigned acc_lo_z)
+  {
+    static_assert(MODE != OutMode::Add, "Add mode needs no initialisation");
+    auto put = [&](int px, int py, int pz) {
+      if ((px == 0 && br.lo_sh[0]) || (py == 0 && br.lo_sh[1]) || (pz == 0 && br.lo_sh[2]))
+        return;
+      if (acc_lo_z && pz == 0 && br.g0[2] == 0)
+        return;
+      const int idx = br.index(px, py, pz);
+      dst[idx]      = (MODE == OutMode::BPlus) ? bvec[idx] : T(0);
+    };
+    constexpr int PX = K * MARCH_BX + 1;
     const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool    mx0 = mask && br.con_lo[0], mx1 = mask && br.con_hi[0];
-    for (int r = warp; r < NR; r += LAY::S::NT / 32)
-      {
-        const int  l = r / PY, py = r % PY, pz = K * lz + l;
-        const bool rowcon = mask && ((br.con_lo[1] && py == 0) || (br.con_hi[1] && py == br.nv[1] - 1) ||
-                                     (br.con_lo[2] && pz == 0) || (br.con_hi[2] && pz == br.nv[2] - 1));
-        const bool rowv    = py < br.nv[1] && pz < br.nv[2] && !rowcon;
-        const int  rowbase = br.g0[0] + br.sy * (br.g0[1] + py) + br.sz * (br.g0[2] + pz);
+    for (int side = br.lo_sh[0] ? 1 : 0; side < 2; ++side)
+      for (int pz = warp; pz < br.nv[2]; pz += MARCH_NT / 32)
+        if (lane < br.nv[1])
+          put(side ? br.nv[0] - 1 : 0, lane, pz);
+    for (int side = br.lo_sh[1] ? 1 : 0; side < 2; ++side)
+      for (int pz = warp; pz < br.nv[2]; pz += MARCH_NT / 32)
 #pragma unroll
         for (int c = 0; c < (PX + 31) / 32; ++c)
-          {
-            const int px = lane + 32 * c;
-            if (px >= PX)
-              break;
-            const bool valid = rowv && px < br.nv[0] && !(mx0 && px == 0) && !(mx1 && px == br.nv[0] - 1);
-            cp_async_elem(buf + r * PX + px, src + (valid ? rowbase + px : 0), valid);
-          }
+          if (lane + 32 * c < br.nv[0])
+            put(lane + 32 * c, side ? br.nv[1] - 1 : 0, pz);
+    for (int side = br.lo_sh[2] ? 1 : 0; side < 2; ++side)
+      for (int py = warp; py < br.nv[1]; py += MARCH_NT / 32)
+#pragma unroll
+        for (int c = 0; c < (PX + 31) / 32; ++c)
+          if (lane + 32 * c < br.nv[0])
+            put(lane + 32 * c, py, side ? br.nv[2] - 1 : 0);
+    __syncthreads();
+    if (threadIdx.x == 0)
+      {
+        __threadfence();
+        st_release(s.flags + br.id, s.epoch);
       }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   }
 
-  // The marching body.  Cell operator: Op::apply(u, valid, cx, cy, cz) in place on (k+1)^3 values.
-  // With DOT the cell operator returns the cell's form src_c^T A_c src_c and the sum over the brick
-  // goes to the fused dot product (release_ticket_dot).
-  template <int K, typename T, OutMode MODE, class Op, bool DOT = false>
+  // Bounded wait of threads 0..6 for the flags of the lower neighbour segments; the caller's next
+  // barrier orders the other threads.
+  template <int K>
+  __device__ __forceinline__ void
+  column_wait_lower(const Column<K> &br, const GridDesc &g, const SyncDesc &s)
+  {
+    if (threadIdx.x < 7)
+      {
+        const unsigned t  = threadIdx.x + 1; // offsets (ox,oy,oz) in {0,1}^3 minus (0,0,0)
+        const int      ox = (t & 1u) ? 1 : 0, oy = (t & 2u) ? 1 : 0, oz = (t & 4u) ? 1 : 0;
+        if ((!ox || br.lo_sh[0]) && (!oy || br.lo_sh[1]) && (!oz || br.lo_sh[2]))
+          {
+            const unsigned nb = br.id - (unsigned)ox - (unsigned)g.nbr[0] * ((unsigned)oy + (unsigned)g.nbr[1] * (unsigned)oz);
+            unsigned       it = 0;
+            while (ld_acquire(s.flags + nb) != s.epoch)
+              {
+                if (++it > s.spin_limit)
+                  {
+                    atomicExch(s.error, ERR_FLAG_WAIT);
+                    break;
+                  }
+                __nanosleep(32);
+              }
+          }
+      }
+  }
+
+  // ---- bulk copies of lattice rows (sm_90+ PTX)
+  __device__ __forceinline__ void
+  march_bar_init(unsigned long long *bar, unsigned count)
+  {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(count)
+                 : "memory");
+  }
+  __device__ __forceinline__ void
+  march_bar_expect(unsigned long long *bar, unsigned bytes)
+  {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)),
+                 "r"(bytes)
+                 : "memory");
+  }
+  // bounded wait for the phase with the given parity (about 2^20 tries, each of which may suspend)
+  __device__ __forceinline__ bool
+  march_bar_wait(unsigned long long *bar, unsigned parity)
+  {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+    for (unsigned it = 0; it < (1u << 20); ++it)
+      {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+        if (ok)
+          return true;
+      }
+    return false;
+  }
+
+  // One lattice row: points [idx, idx + n) of src (n_src points in all) into the slot row, shifted by the
+  // row's misalignment; the caller has computed base = src's own misalignment in elements.  Returns the
+  // bytes copied in bulk.  issue = false only returns them.
+  template <typename T>
+  __device__ __forceinline__ unsigned
+  march_row(const T *src, int n_src, int base, int idx, int n, T *slot, unsigned long long *bar, bool issue)
+  {
+    constexpr int G  = 16 / (int)sizeof(T);
+    const int     sh = (base + idx) & (G - 1), first = idx - sh, len = (sh + n + G - 1) / G * G;
+    const int     beg = first < 0 ? G : 0, end = (long long)first + len > n_src ? len - G : len;
+    const unsigned bytes = end > beg ? (unsigned)((end - beg) * (int)sizeof(T)) : 0u;
+    if (issue)
+      {
+        if (bytes)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(slot + beg)),
+                       "l"(src + (first + beg)), "r"(bytes), "r"((unsigned)__cvta_generic_to_shared(bar))
+                       : "memory");
+      }
+    else
+      {
+        // granules that reach outside the vector, point by point
+        if (beg)
+          for (int i = sh; i < min(G, sh + n); ++i)
+            slot[i] = src[first + i];
+        if (end < len && !(beg && len == G))
+          for (int i = max(end, sh); i < sh + n; ++i)
+            slot[i] = src[first + i];
+      }
+    return bytes;
+  }
+
+  // Warp 0: the planes [p0, p1) of the segment into their ring slots (slot = plane mod NRING); every
+  // lane arrives on the barrier once (count 32), with the bytes of its rows.
+  template <int K, typename T>
+  __device__ __forceinline__ void
+  march_stage(const Column<K> &br, const T *src, int n_src, int base, int p0, int p1, T *ring, unsigned long long *bar)
+  {
+    using LAY = MarchLayout<K, T>;
+    const int lane = threadIdx.x;
+    const int rows = (p1 - p0) * LAY::PY;
+    auto      row  = [&](int r, bool issue) -> unsigned {
+      const int py = r % LAY::PY, pz = p0 + r / LAY::PY;
+      if (py >= br.nv[1] || pz >= br.nv[2])
+        return 0u;
+      return march_row<T>(src, n_src, base, br.index(0, py, pz), br.nv[0],
+                          ring + (pz % LAY::NRING) * LAY::PLANE + py * LAY::PITCH, bar, issue);
+    };
+    unsigned bytes = 0;
+    for (int r = lane; r < rows; r += 32)
+      bytes += row(r, false);
+    // the slots were read by every thread before the CTA's last barrier; order those reads before the
+    // copies of the asynchronous proxy
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    march_bar_expect(bar, bytes);
+    for (int r = lane; r < rows; r += 32)
+      row(r, true);
+  }
+
+  // The marching body.  Cell operator: op.apply<DOT>(u, op.load(valid, cx, cy, cz)) in place on (K+1)^3 values.
+  // With DOT the cell operator returns the cell's form src_c^T A src_c and the sum over the segment goes
+  // to the fused dot product (release_ticket_dot).
+  // MASKABLE: the operator may carry per-DoF constraint flags (GridDesc::cmask) besides the faces.
+  template <int K, typename T, OutMode MODE, class Op, bool DOT = false, bool MASKABLE = false>
   __device__ __forceinline__ void
   march_body(const GridDesc &g, const SyncDesc &s, const T *src, T *dst, const T *bvec, bool mask_src, const Op &op,
-             T *smem, unsigned *s_ticket, const DotSink &dot = DotSink{}, double *s_red = nullptr)
+             T *smem, unsigned *s_ticket, unsigned long long *bars, const DotSink &dot = DotSink{},
+             double *s_red = nullptr)
   {
     double dsum = 0.0;
-    using LAY       = MarchLayout<K, T>;
-    using BR        = typename LAY::BR;
-    constexpr int N = K + 1, PX = LAY::PX, PY = LAY::PY, BZ = LAY::S::BZ;
-    T *buf0 = smem, *buf1 = smem + LAY::LAYER, *yx = smem + 2 * LAY::LAYER;
+    using LAY   = MarchLayout<K, T>;
+    constexpr int N = K + 1, G = LAY::G, PITCH = LAY::PITCH, NRING = LAY::NRING;
+    T *ring = smem, *yx0 = smem + NRING * LAY::PLANE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    BR        br;
-    if (!brick_begin<BR, T, MODE>(br, g, s, dst, bvec, s_ticket))
-      return;
+    Column<K> br;
+    if (threadIdx.x == 0)
+      {
+        march_bar_init(&bars[0], 32);
+        march_bar_init(&bars[1], 32);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      }
     if constexpr (MODE != OutMode::Add)
-      if (br.has_lower_neighbour())
-        brick_wait_lower(br, g, s);
+      {
+        const unsigned t = take_ticket(s, s_ticket);
+        if (t >= (unsigned)(g.nbr[0] * g.nbr[1] * g.nbr[2]))
+          {
+            // stale counter: never index past the flag array; report and keep the count
+            if (threadIdx.x == 0)
+              atomicExch(s.error, ERR_TICKET);
+            release_ticket(s);
+            return;
+          }
+        br.set(g, t);
+      }
+    else
+      {
+        br.set(g, blockIdx.x);
+        __syncthreads(); // barriers initialised
+      }
+    const int n_src = g.n[0] * g.n[1] * g.n[2];
+    const int base  = (int)((reinterpret_cast<unsigned long long>(src) / sizeof(T)) & (G - 1));
+    const int nlayers = br.layers;
+    if (warp == 0)
+      {
+        march_stage<K, T>(br, src, n_src, base, 0, K + 1, ring, &bars[0]);
+        if (nlayers > 1)
+          march_stage<K, T>(br, src, n_src, base, K + 1, 2 * K + 1, ring, &bars[1]);
+      }
+    if constexpr (MODE != OutMode::Add)
+      column_init_publish<K, T, MODE>(br, s, dst, bvec, g.acc_lo_z);
     const int  cx = br.c0[0] + lane, cy = br.c0[1] + warp;
     const bool vxy       = cx < g.m[0] && cy < g.m[1];
-    const bool last_lane = cx == min(br.c0[0] + 32, g.m[0]) - 1;
-    const bool last_warp = cy == min(br.c0[1] + 4, g.m[1]) - 1;
-    const int  nlayers   = min(BZ, g.m[2] - br.c0[2]);
-    const bool do_mask   = mask_src && br.any_con; // only bricks on a constrained face pay for masking
-    // flags: x / y faces shared with the lower neighbour columns, Dirichlet planes through the cell
-    const bool cI0 = br.con_lo[0] && cx == 0, cIK = br.con_hi[0] && K * cx + K == g.n[0] - 1;
-    const bool cJ0 = br.con_lo[1] && cy == 0, cJK = br.con_hi[1] && K * cy + K == g.n[1] - 1;
-    T carry[N * N];
+    const bool last_lane = cx == min(br.c0[0] + MARCH_BX, g.m[0]) - 1;
+    const bool last_warp = cy == min(br.c0[1] + MARCH_BY, g.m[1]) - 1;
+    const bool do_mask   = mask_src && br.any_con; // only segments on a constrained face pay for masking
+    // Dirichlet planes through the cell
+    const bool cI0 = br.con_lo[0] && cx == 0, cIK = br.con_hi[0] && cx == g.m[0] - 1;
+    const bool cJ0 = br.con_lo[1] && cy == 0, cJK = br.con_hi[1] && cy == g.m[1] - 1;
+    T carry[K * K];
 #pragma unroll
-    for (int q = 0; q < N * N; ++q)
+    for (int q = 0; q < K * K; ++q)
       carry[q] = T(0);
-    const int cbase0 = (br.g0[0] + K * lane) + br.sy * (br.g0[1] + K * warp) + br.sz * br.g0[2];
-    march_stage<LAY>(br, 0, src, do_mask, buf0);
+    const int wbase  = br.index(0, K * warp, 0); // first point of the warp's cell row
+    int       slot0  = 0;                          // ring slot of the layer's low plane
     for (int lz = 0; lz < nlayers; ++lz)
       {
-        T *cur = (lz & 1) ? buf1 : buf0;
-        if (lz + 1 < nlayers)
-          {
-            march_stage<LAY>(br, lz + 1, src, do_mask, (lz & 1) ? buf0 : buf1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-          }
-        else
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+        // lanes outside the mesh compute on whatever the slot holds: their values only reach lanes and
+        // warps outside the mesh, too
+        const int  cz  = br.c0[2] + lz;
+        const auto pre = op.load(vxy, cx, cy, cz); // per-cell coefficients, in flight during the wait
+        if (!march_bar_wait(&bars[lz & 1], (unsigned)(lz >> 1) & 1u) && lane == 0)
+          atomicExch(s.error, ERR_FLAG_WAIT);
         const bool last_layer = lz == nlayers - 1;
-        const int  cz         = br.c0[2] + lz;
+        const bool cL0 = br.con_lo[2] && cz == 0, cLK = br.con_hi[2] && cz == g.m[2] - 1;
         T          u[N * N * N];
 #pragma unroll
         for (int l = 0; l < N; ++l)
+          {
+            int sl = slot0 + l;
+            if (sl >= NRING)
+              sl -= NRING;
+            const T *pl = ring + sl * LAY::PLANE + (K * warp) * PITCH + K * lane;
+            const int e = base + wbase + br.sz * (K * lz + l);
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+            for (int j = 0; j < N; ++j)
+              {
+                const T *row = pl + j * PITCH + ((e + j * br.sy) & (G - 1));
 #pragma unroll
-            for (int i = 0; i < N; ++i)
-              u[(l * N + j) * N + i] = vxy ? cur[(l * PY + K * warp + j) * PX + K * lane + i] : T(0);
+                for (int i = 0; i < N; ++i)
+                  u[(l * N + j) * N + i] = row[i];
+              }
+          }
+        slot0 += K;
+        if (slot0 >= NRING)
+          slot0 -= NRING;
+        if (do_mask)
+          {
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+#pragma unroll
+              for (int j = 0; j < N; ++j)
+                {
+                  const bool cr = (l == 0 && cL0) || (l == K && cLK) || (j == 0 && cJ0) || (j == K && cJK);
+#pragma unroll
+                  for (int i = 0; i < N; ++i)
+                    if (cr || (i == 0 && cI0) || (i == K && cIK))
+                      u[(l * N + j) * N + i] = T(0);
+                }
+          }
+        if constexpr (MASKABLE)
+          if (g.cmask != nullptr && mask_src && vxy)
+            {
+              const uint8_t *cm = g.cmask + (wbase + K * lane + br.sz * (K * lz));
+#pragma unroll
+              for (int l = 0; l < N; ++l)
+#pragma unroll
+                for (int j = 0; j < N; ++j)
+#pragma unroll
+                  for (int i = 0; i < N; ++i)
+                    if (cm[j * br.sy + l * br.sz + i])
+                      u[(l * N + j) * N + i] = T(0);
+            }
         if constexpr (DOT)
-          dsum += op.template apply<true>(u, vxy, cx, cy, cz);
+          dsum += vxy ? op.template apply<true>(u, pre) : 0.0;
         else
-          op.template apply<false>(u, vxy, cx, cy, cz);
-        // x: lane t adds lane t-1's x = K face; only the last lane keeps its own
+          op.template apply<false>(u, pre);
+        // x: lane t adds lane t-1's x = K face
 #pragma unroll
         for (int q = 0; q < N * N; ++q)
           {
             const T v = __shfl_up_sync(0xffffffffu, u[q * N + K], 1);
             if (lane > 0)
               u[q * N] += v;
-            if (!last_lane)
-              u[q * N + K] = T(0);
           }
-        // y: warp w adds warp w-1's y = K face; only the last warp keeps its own
+        // y: warp w hands its y = K face to warp w + 1 (the last warp adds its own to dst below)
+        T *yx = yx0 + (lz & 1) * LAY::YX;
 #pragma unroll
         for (int l = 0; l < N; ++l)
 #pragma unroll
-          for (int i = 0; i < N; ++i)
-            yx[((warp * N + l) * N + i) * 32 + lane] = u[(l * N + K) * N + i];
+          for (int i = 0; i < K; ++i)
+            yx[((warp * N + l) * K + i) * 32 + lane] = u[(l * N + K) * N + i];
+        if constexpr (MODE != OutMode::Add)
+          if (lz == 0 && br.has_lower_neighbour())
+            column_wait_lower<K>(br, g, s);
         __syncthreads();
+        // every thread has read the layer's planes: those that the layer after next needs not are free
+        if (warp == 0 && lz + 2 < nlayers)
+          march_stage<K, T>(br, src, n_src, base, K * (lz + 2) + 1, K * (lz + 3) + 1, ring, &bars[lz & 1]);
         if (warp > 0)
 #pragma unroll
           for (int l = 0; l < N; ++l)
 #pragma unroll
-            for (int i = 0; i < N; ++i)
-              u[(l * N) * N + i] += yx[(((warp - 1) * N + l) * N + i) * 32 + lane];
-        if (!last_warp)
-#pragma unroll
-          for (int l = 0; l < N; ++l)
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-              u[(l * N + K) * N + i] = T(0);
+            for (int i = 0; i < K; ++i)
+              u[(l * N) * N + i] += yx[(((warp - 1) * N + l) * K + i) * 32 + lane];
         // z: add the carried face, carry this layer's z = K face
 #pragma unroll
-        for (int q = 0; q < N * N; ++q)
-          {
-            u[q] += carry[q];
-            carry[q] = u[K * N * N + q];
-          }
-        // ---- write-out.  Every brick-face point was initialised by its owner (brick_init_publish),
-        // so a face point is an atomic add (skipped on constrained rows) and an interior point a
-        // plain store; interior points are never constrained (Dirichlet planes are domain faces).
-        if (vxy)
-          {
-            const int  cbase = cbase0 + br.sz * (K * lz);
-            const bool f_x0 = lane == 0, f_y0 = warp == 0, f_z0 = lz == 0;
-            const bool cL0 = br.con_lo[2] && cz == 0, cLK = br.con_hi[2] && K * cz + K == g.n[2] - 1;
-#define MPDG_PUT(i, j, l)                                                                                      \
-  {                                                                                                            \
-    const int idx_ = cbase + (j) * br.sy + (l) * br.sz + (i);                                                  \
-    const T   v_   = u[((l) * N + (j)) * N + (i)];                                                             \
-    const bool face_ = ((i) == 0 && f_x0) || (i) == K || ((j) == 0 && f_y0) || (j) == K || ((l) == 0 && f_z0) || \
-                       (l) == K;                                                                               \
-    if (face_)                                                                                                 \
-      {                                                                                                        \
-        const bool cn_ = ((i) == 0 && cI0) || ((i) == K && cIK) || ((j) == 0 && cJ0) || ((j) == K && cJK) ||    \
-                         ((l) == 0 && cL0) || ((l) == K && cLK);                                               \
-        if (!cn_)                                                                                              \
-          atomicAdd(dst + idx_, v_);                                                                           \
-      }                                                                                                        \
-    else if constexpr (MODE == OutMode::Set)                                                                   \
-      dst[idx_] = v_;                                                                                          \
-    else if constexpr (MODE == OutMode::Add)                                                                   \
-      dst[idx_] += v_;                                                                                         \
-    else                                                                                                       \
-      dst[idx_] = bvec[idx_] + v_;                                                                             \
-  }
+        for (int j = 0; j < K; ++j)
+#pragma unroll
+          for (int i = 0; i < K; ++i)
+            {
+              u[j * N + i] += carry[j * K + i];
+              carry[j * K + i] = u[(K * N + j) * N + i];
+            }
+        // ---- write-out.  Every face point of the segment was initialised by its owner
+        // (column_init_publish), so a face point is an atomic add (skipped on constrained rows) and an
+        // interior point a plain store; interior points are never constrained (Dirichlet planes are
+        // domain faces).
+        auto write_out = [&](auto flagged) {
+            constexpr bool CM    = decltype(flagged)::value;
+            const int      cbase = wbase + K * lane + br.sz * (K * lz);
+            T             *d0    = dst + cbase;
+            const bool     x_low = lane == 0;
+            auto store = [&](int i, int j, int l) {
+              const int off = j * br.sy + l * br.sz + i;
+              const T   v   = u[(l * N + j) * N + i];
+              bool con = false;
+              if constexpr (CM)
+                con = g.cmask[cbase + off] != 0;
+              if constexpr (MODE == OutMode::Set)
+                d0[off] = con ? T(0) : v;
+              else if constexpr (MODE == OutMode::Add)
+                {
+                  if (!con)
+                    d0[off] += v;
+                }
+              else
+                d0[off] = con ? bvec[cbase + off] : bvec[cbase + off] + v;
+            };
+            auto add = [&](int i, int j, int l) {
+              const int off = j * br.sy + l * br.sz + i;
+              if constexpr (CM)
+                if (g.cmask[cbase + off])
+                  return;
+              atomicAdd(d0 + off, u[(l * N + j) * N + i]);
+            };
 #pragma unroll
             for (int l = 0; l < K; ++l)
 #pragma unroll
               for (int j = 0; j < K; ++j)
+                {
+                  if ((j == 0 && warp == 0) || (l == 0 && lz == 0))
+                    {
+                      if (!((j == 0 && cJ0) || (l == 0 && cL0)))
 #pragma unroll
-                for (int i = 0; i < K; ++i)
-                  MPDG_PUT(i, j, l)
-            if (last_lane)
+                        for (int i = 0; i < K; ++i)
+                          if (!(i == 0 && cI0))
+                            add(i, j, l);
+                    }
+                  else
+                    {
+                      if (!x_low)
+                        store(0, j, l);
+#pragma unroll
+                      for (int i = 1; i < K; ++i)
+                        store(i, j, l);
+                    }
+                }
+            if (x_low && !cI0)
 #pragma unroll
               for (int l = 0; l < K; ++l)
 #pragma unroll
                 for (int j = 0; j < K; ++j)
-                  MPDG_PUT(K, j, l)
-            if (last_warp)
+                  if (!((j == 0 && warp == 0) || (l == 0 && lz == 0)))
+                    add(0, j, l);
+            if (last_lane && !cIK)
 #pragma unroll
-              for (int l = 0; l < K; ++l)
+              for (int l = 0; l < N; ++l)
 #pragma unroll
-                for (int i = 0; i < N; ++i)
-                  if (i < K || last_lane)
-                    MPDG_PUT(i, K, l)
-            if (last_layer)
+                for (int j = 0; j < N; ++j)
+                  if (!((j == 0 && cJ0) || (j == K && cJK) || (l == 0 && cL0) || (l == K && cLK)))
+                    add(K, j, l);
+            if (last_warp && !cJK)
 #pragma unroll
-              for (int j = 0; j < N; ++j)
+              for (int l = 0; l < N; ++l)
+                if (!((l == 0 && cL0) || (l == K && cLK)))
 #pragma unroll
-                for (int i = 0; i < N; ++i)
-                  if ((i < K || last_lane) && (j < K || last_warp))
-                    MPDG_PUT(i, j, K)
-#undef MPDG_PUT
+                  for (int i = 0; i < K; ++i)
+                    if (!(i == 0 && cI0))
+                      add(i, K, l);
+            if (last_layer && !cLK)
+#pragma unroll
+              for (int j = 0; j < K; ++j)
+                if (!(j == 0 && cJ0))
+#pragma unroll
+                  for (int i = 0; i < K; ++i)
+                    if (!(i == 0 && cI0))
+                      add(i, j, K);
+        };
+        if (vxy)
+          {
+            if constexpr (MASKABLE)
+              {
+                if (g.cmask != nullptr)
+                  write_out(std::true_type());
+                else
+                  write_out(std::false_type());
+              }
+            else
+              write_out(std::false_type());
           }
-        // no barrier here: the next layer's cp.async staging overwrites the buffer every thread
-        // finished reading before this layer's y-exchange barrier, and the next y-exchange writes
-        // come after the next layer's first barrier
       }
     if constexpr (DOT)
-      release_ticket_dot<LAY::S::NT>(s, dot, br.id, dsum, s_red, s_ticket);
+      release_ticket_dot<MARCH_NT>(s, dot, br.id, dsum, s_red, s_ticket);
     else if constexpr (MODE != OutMode::Add)
       release_ticket(s);
   }

@@ -6,6 +6,7 @@
 // cudaMalloc, cudaFree or any routine that allocates device memory.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 #include <string>
@@ -120,7 +121,8 @@ mpdg_heat_vmult_noalloc(const mpdg_mesh_desc *mesh, const mpdg_op_params *params
     return reject(MPDG_ERR_CUDA, std::string("cudaGetSymbolAddress of the scratch array: ") + cudaGetErrorString(e));
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   // ticket, done, error word and this mesh's flags must start at zero (epoch 1 marks "initialised")
-  e = cudaMemsetAsync(scratch, 0, sizeof(unsigned) * (kFlagWordStart + nbrk), stream);
+  const long long flags = std::min<long long>(heat_flags(mesh->degree, g.m, true), MPDG_NOALLOC_MAX_BRICKS);
+  e = cudaMemsetAsync(scratch, 0, sizeof(unsigned) * (kFlagWordStart + flags), stream);
   if (e != cudaSuccess)
     return reject(MPDG_ERR_CUDA, std::string("clearing the scratch array: ") + cudaGetErrorString(e));
 
