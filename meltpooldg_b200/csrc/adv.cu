@@ -7,17 +7,20 @@
 // The velocity is an affine field v(x) = v0 + G x evaluated analytically at the Gauss points (the
 // reference evaluates a dealii::Function there, :475-479); rigid rotations are affine.
 //
-// Per cell (one thread), FEEvaluation-style sum factorisation in registers:
-//   u_q = (B(x)B(x)B) u;  for d: g = D_d u_q (collocation derivative on the Gauss points),
-//   R += JxW theta v_d g / h_d,  R += D_d^T (JxW theta eps g / h_d^2);  out = (B(x)B(x)B)^T R,
-// starting from R = JxW u_q / dt.  Peak register use is three cell arrays (u_q, R, g).
+// Per cell (one thread), sum factorisation in registers on the Gauss points, in the column-marching
+// frame of march.cuh.  With u_q = (B(x)B(x)B) u the operator's values are kept without the point weights,
+//   S = u_q / dt + sum_d [ v_d (theta D_d / h_d) u_q + L_d u_q ],   L_d = theta eps / h_d^2 W^-1 D^T W D
+// (D the 1-D collocation derivative on the Gauss points, W its weights), so that a point costs one addition
+// for its velocity and one fused multiply-add, and out = (B^T W (x) B^T W (x) B^T W) S.  For an affine velocity
+// v_d at a point is the cell's value plus three per-direction offsets.  D, L and E act on the differences of
+// neighbouring values (gausspoint.cuh).
 //
 // SUPG (ConvectionStabilizationType::SUPG, :455-457, :486-490, stabilisation parameter :497-533):
-// the strong residual s = u/dt + theta v.grad u - theta eps lap u at the Gauss points (the second
-// derivative is the collocation derivative applied twice: exact for the degree-k interpolant), tested
-// with tau_c v.grad phi; tau_c = (coefficient < 0 ? 1 / max_q |v| (0 below 1e-6) : coefficient) times
-// the cell size diameter / sqrt(3) (source/core/scratch_data.cpp:262-277).  The rhs uses the same
-// form with theta replaced by theta - 1 (:322-345).
+// the strong residual s = u/dt + theta v.grad u - theta eps lap u at the Gauss points (E_d = theta eps /
+// h_d^2 D D: exact for the degree-k interpolant), tested with tau_c v.grad phi; tau_c = (coefficient < 0 ?
+// 1 / max_q |v| (0 below 1e-6) : coefficient) times the cell size diameter / sqrt(3)
+// (source/core/scratch_data.cpp:262-277).  The rhs uses the same form with theta replaced by theta - 1
+// (:322-345).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,50 +29,13 @@
 #include <set>
 
 #include "brick.cuh"
+#include "gausspoint.cuh"
 #include "kernels.h"
-#include "sumfac.cuh"
+#include "march.cuh"
 
 namespace mpdg
 {
-  // Per degree (1..3) in constant memory, uploaded once per device:
-  //   [B (n*n): phi_i(x_q) | D (n*n): collocation derivative on the Gauss points |
-  //    qp (n): Gauss points | qw3 (n^3): tensor Gauss weights]
   constexpr int ADV_KMAX = 3;
-  constexpr int ADV_TAB  = 2 * 16 + 4 + 64;
-  __constant__ double c_adv_d[ADV_KMAX + 1][ADV_TAB];
-  __constant__ float  c_adv_f[ADV_KMAX + 1][ADV_TAB];
-
-  template <typename T>
-  __device__ __forceinline__ const T *
-  adv_table(int K)
-  {
-    if constexpr (sizeof(T) == 8)
-      return c_adv_d[K];
-    else
-      return c_adv_f[K];
-  }
-
-  template <typename T, int N>
-  struct AdvArgs
-  {
-    T            det;
-    T            supg_coef, cell_size;
-    GridDesc     g;
-    SyncDesc     s;
-    T            inv_dt, th_adv, th_dif; // already multiplied by scale
-    T            vel[12];
-    T            origin[3], h[3];
-    const T     *src;
-    T           *dst;
-    const T     *b;
-    int          mask_src;
-    const int   *skip;
-    const double *vfield[3]; // velocity as a DoF vector (three FE_Q(k) components), else affine
-    // cell-independent factors per direction d and Gauss point q (N^3 <= 27 used):
-    //   pa = th_adv det / h_d w_q,  pb = pa (G_d. (h (x) qp_q)),  pd = th_dif det / h_d^2 w_q;
-    // pm = det inv_dt w_q.  The velocity term of a cell is (vd0 pa + pb) g, vd0 = v_d(cell origin).
-    T pa[3][64], pb[3][64], pd[3][64], pm[64];
-  };
 
   // out = M in along a line (in place), M[a*N+b], TR: transpose
   template <typename T, int N, int S, bool TR>
@@ -91,22 +57,6 @@ namespace mpdg
       }
   }
 
-  // acc += M^T g along a line
-  template <typename T, int N, int S>
-  __device__ __forceinline__ void
-  line_mat_tr_acc(T *acc, const T *g, const int base, const T *M)
-  {
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-      {
-        T s = acc[base + a * S];
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-          s = fma(M[k * N + a], g[base + k * S], s);
-        acc[base + a * S] = s;
-      }
-  }
-
   template <typename T, int N, int D, bool TR>
   __device__ __forceinline__ void
   sweep(T *v, const T *M)
@@ -119,142 +69,6 @@ namespace mpdg
         {
           const int base = D == 0 ? (a * N + c) * N : (D == 1 ? a * N * N + c : a * N + c);
           line_mat<T, N, S, TR>(v, base, M);
-        }
-  }
-
-  template <typename T, int N, int D>
-  __device__ __forceinline__ void
-  sweep_tr_acc(T *acc, const T *g, const T *M)
-  {
-    constexpr int S = D == 0 ? 1 : (D == 1 ? N : N * N);
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-      for (int c = 0; c < N; ++c)
-        {
-          const int base = D == 0 ? (a * N + c) * N : (D == 1 ? a * N * N + c : a * N + c);
-          line_mat_tr_acc<T, N, S>(acc, g, base, M);
-        }
-  }
-
-  // One direction d of the advection and diffusion terms, line by line (a line along d at a time):
-  //   g = D_d uq along the line;  R += theta_adv v_d JxW g / h_d;  R += D_d^T (theta_dif JxW g / h_d^2)
-  // with the cell-independent factors of each point precomputed (AdvArgs::pa, pb, pd): the velocity
-  // weight is vd0 pa_q + pb_q (affine field) or vq_q pa_q (DoF-vector field).  Only the k+1 values of
-  // one line are live besides uq and R.
-  template <typename T, int N, int D>
-  __device__ __forceinline__ void
-  adv_direction(const T *uq, T *R, const T *tD, const T *pa, const T *pb, const T *pd, T vd0, bool dif,
-                const T *vq = nullptr)
-  {
-    constexpr int S = D == 0 ? 1 : (D == 1 ? N : N * N);
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-      for (int c = 0; c < N; ++c)
-        {
-          const int base = D == 0 ? (a * N + c) * N : (D == 1 ? a * N * N + c : a * N + c);
-          T         g[N];
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              T s = tD[r * N] * uq[base];
-#pragma unroll
-              for (int k = 1; k < N; ++k)
-                s = fma(tD[r * N + k], uq[base + k * S], s);
-              g[r] = s;
-            }
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              const int q = base + r * S;
-              const T   w = vq ? vq[q] * pa[q] : fma(vd0, pa[q], pb[q]);
-              R[q]        = fma(w, g[r], R[q]);
-              g[r] *= pd[q];
-            }
-          if (dif)
-#pragma unroll
-            for (int r = 0; r < N; ++r)
-              {
-                T s = R[base + r * S];
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                  s = fma(tD[k * N + r], g[k], s);
-                R[base + r * S] = s;
-              }
-        }
-  }
-
-  // SUPG, direction D of the strong residual: s += theta_adv v_d (D_d u_q) / h_d - theta_dif (D_d D_d u_q) / h_d^2
-  // (v_d from the affine field, or vq = v_d at the Gauss points of a DoF-vector field)
-  template <typename T, int N, int D>
-  __device__ __forceinline__ void
-  supg_residual(const T *uq, T *sres, const T *tD, const T *tqp, T inv_h, T vd0, T gx, T gy, T gz, T th_adv,
-                T th_dif, const T *vq = nullptr)
-  {
-    constexpr int S = D == 0 ? 1 : (D == 1 ? N : N * N);
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-      for (int c = 0; c < N; ++c)
-        {
-          const int base = D == 0 ? (a * N + c) * N : (D == 1 ? a * N * N + c : a * N + c);
-          T         g[N];
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              T s = tD[r * N] * uq[base];
-#pragma unroll
-              for (int k = 1; k < N; ++k)
-                s = fma(tD[r * N + k], uq[base + k * S], s);
-              g[r] = s;
-            }
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              T gg = tD[r * N] * g[0];
-#pragma unroll
-              for (int k = 1; k < N; ++k)
-                gg = fma(tD[r * N + k], g[k], gg);
-              const int q  = base + r * S;
-              const int qx = q % N, qy = (q / N) % N, qz = q / (N * N);
-              const T   vd = vq ? vq[q] : vd0 + gx * tqp[qx] + gy * tqp[qy] + gz * tqp[qz];
-              sres[q] += th_adv * vd * g[r] * inv_h - th_dif * gg * inv_h * inv_h;
-            }
-        }
-  }
-
-  // SUPG, direction D of the test with tau v.grad phi: R += D_d^T (c_t w3 v_d s), c_t = tau det / h_d
-  template <typename T, int N, int D>
-  __device__ __forceinline__ void
-  supg_test(const T *sres, T *R, const T *tD, const T *tqp, const T *tw3, T c_t, T vd0, T gx, T gy, T gz,
-            const T *vq = nullptr)
-  {
-    constexpr int S = D == 0 ? 1 : (D == 1 ? N : N * N);
-#pragma unroll
-    for (int a = 0; a < N; ++a)
-#pragma unroll
-      for (int c = 0; c < N; ++c)
-        {
-          const int base = D == 0 ? (a * N + c) * N : (D == 1 ? a * N * N + c : a * N + c);
-          T         t[N];
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              const int q  = base + r * S;
-              const int qx = q % N, qy = (q / N) % N, qz = q / (N * N);
-              const T   vd = vq ? vq[q] : vd0 + gx * tqp[qx] + gy * tqp[qy] + gz * tqp[qz];
-              t[r]         = c_t * tw3[q] * vd * sres[q];
-            }
-#pragma unroll
-          for (int r = 0; r < N; ++r)
-            {
-              T s = R[base + r * S];
-#pragma unroll
-              for (int k = 0; k < N; ++k)
-                s = fma(tD[k * N + r], t[k], s);
-              R[base + r * S] = s;
-            }
         }
   }
 
@@ -289,38 +103,6 @@ namespace mpdg
     return tau * cell_size;
   }
 
-#ifndef MPDG_ADV_MINB_F64
-#define MPDG_ADV_MINB_F64 2
-#endif
-#ifndef MPDG_ADV_MINB_F32
-#define MPDG_ADV_MINB_F32 4
-#endif
-
-  template <int K, typename T>
-  struct AdvLayout
-  {
-    static constexpr int  N  = K + 1;
-    static constexpr int  BX = 8, BY = 8, BZ = (K == 1 ? 8 : (K == 2 ? 4 : 2));
-    static constexpr int  NT = BX * BY * BZ;
-    using BR                 = Brick<K, BX, BY, BZ, NT>;
-    static constexpr size_t bytes = sizeof(T) * 2 * (size_t)BR::NPTS; // staged input + accumulator
-    // SUPG with a DoF-vector velocity at k <= 2: the velocity's three components staged as well
-    static constexpr bool   STAGE_FIELD  = K <= 2;
-    static constexpr size_t bytes_staged = bytes + sizeof(double) * 3 * (size_t)BR::NPTS;
-    // CTAs per SM (k = 3: two CTAs of 128 threads, so that the two 64-value cell arrays fit registers)
-    static constexpr int    MINB  = K == 3 ? 2 : (sizeof(T) == 8 ? MPDG_ADV_MINB_F64 : MPDG_ADV_MINB_F32);
-  };
-
-  // The SUPG form keeps a third cell array (the strong residual).  At k = 2 it is held to half the
-  // CTAs per SM of the plain form (at least one); at k = 1 the arrays are small and the plain
-  // occupancy wins despite some spilling (Q1 FP64: 658 against 988 us per 7.2 M DoFs).
-  template <int K, typename T, bool SUPG>
-  struct AdvMinBlocks
-  {
-    static constexpr int value =
-      (SUPG && K == 2) ? (AdvLayout<K, T>::MINB > 1 ? AdvLayout<K, T>::MINB / 2 : 1) : AdvLayout<K, T>::MINB;
-  };
-
   // Velocity component d of a DoF-vector field at the cell's Gauss points: the cell's nodal values
   // read plainly (advection_diffusion_operator.cpp:461-466), interpolated by three sweeps of B.
   template <typename T, int N>
@@ -341,246 +123,258 @@ namespace mpdg
     sweep<T, N, 2, false>(vq, tB);
   }
 
-  // The same from the brick's staged copy of the component (cell's first point at brick index base)
-  template <typename T, int N, int PX, int PY>
-  __device__ __forceinline__ void
-  field_at_points_staged(const double *sf, int base, const T *tB, T *vq)
+  // Kernel parameters of the apply; the 1-D matrices are row-major N x N (point first).
+  template <typename T, int N>
+  struct AdvArgs
   {
+    GridDesc      g;
+    SyncDesc      s;
+    const T      *src;
+    T            *dst;
+    const T      *b;
+    int           mask_src, dif;
+    const int    *skip;
+    const double *vfield[3];  // velocity as a DoF vector (three FE_Q(k) components), else affine
+    T             B[N * N];   // nodal values -> Gauss points
+    T             Bt[3][N * N]; // tests back to the nodes per direction, weighted (rows: nodes); det in [2]
+    T             mass;         // scale / dt
+    // on the differences of neighbouring values (N x (N - 1)), times scale:
+    T             D[3][N * (N - 1)]; // theta / h_d D
+    T             L[3][N * (N - 1)]; // theta eps / h_d^2 W^-1 D^T W D
+    T             E[3][N * (N - 1)]; // SUPG: theta eps / h_d^2 D D
+    T             P[3][N * N];       // SUPG: W^-1 D^T W / h_d
+    double        vel[12], origin[3], h[3]; // affine velocity: the cell's value in double, rounded once
+    T             voff[3][3][N];   // v_d at the Gauss points minus v_d at the cell's origin, per direction
+    T             supg_coef, cell_size;
+  };
+
+  // One direction of the operator, line by line on the differences of u: g = D u, S += v g + L u, and with
+  // SUPG s += v g - E u.  FIRST: S and s start from mass u.  vel(q): the velocity component at point q.
+  template <typename T, int N, int DIR, bool FIRST, bool SUPG, class Vel>
+  __device__ __forceinline__ void
+  adv_direction(const T *u, T *S, T *s, const T *D, const T *L, const T *E, T mass, bool dif, const Vel &vel)
+  {
+    constexpr int ST = DIR == 0 ? 1 : (DIR == 1 ? N : N * N), ND = N - 1;
 #pragma unroll
-    for (int l = 0; l < N; ++l)
+    for (int a = 0; a < N; ++a)
 #pragma unroll
-      for (int j = 0; j < N; ++j)
+      for (int c = 0; c < N; ++c)
+        {
+          const int b = DIR == 0 ? (a * N + c) * N : (DIR == 1 ? a * N * N + c : a * N + c);
+          T         du[ND];
 #pragma unroll
-        for (int i = 0; i < N; ++i)
-          vq[(l * N + j) * N + i] = (T)sf[base + l * PY * PX + j * PX + i];
-    sweep<T, N, 0, false>(vq, tB);
-    sweep<T, N, 1, false>(vq, tB);
-    sweep<T, N, 2, false>(vq, tB);
+          for (int k = 0; k < ND; ++k)
+            du[k] = u[b + (k + 1) * ST] - u[b + k * ST];
+#pragma unroll
+          for (int r = 0; r < N; ++r)
+            {
+              const int q = b + r * ST;
+              T         g = D[r * ND] * du[0];
+#pragma unroll
+              for (int k = 1; k < ND; ++k)
+                g = fma(D[r * ND + k], du[k], g);
+              const T v = vel(q), from = FIRST ? mass * u[q] : S[q];
+              S[q]      = fma(v, g, from);
+              if constexpr (SUPG)
+                s[q] = FIRST ? S[q] : fma(v, g, s[q]);
+            }
+          if (dif)
+#pragma unroll
+            for (int r = 0; r < N; ++r)
+#pragma unroll
+              for (int k = 0; k < ND; ++k)
+                {
+                  const int q = b + r * ST;
+                  S[q]        = fma(L[r * ND + k], du[k], S[q]);
+                  if constexpr (SUPG)
+                    s[q] = fma(-E[r * ND + k], du[k], s[q]);
+                }
+        }
   }
 
-  // SUPG = true: the stabilised form; VDOF = true: the velocity is a DoF vector (three cell arrays
-  // live in both cases; the DoF-vector form keeps the plain form's occupancy and spills, measured
-  // faster than half the CTAs per SM: 287 against 375 us FP64, 194 against 216 us FP32 on 96^3 k = 2)
-  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF = false>
-  __global__ void __launch_bounds__(AdvLayout<K, T>::BR::NT, AdvMinBlocks<K, T, SUPG>::value)
-  adv_apply_kernel(const __grid_constant__ AdvArgs<T, K + 1> a)
+  template <int K, typename T, bool SUPG, bool VDOF>
+  struct AdvCellOp
   {
-    using LAY             = AdvLayout<K, T>;
-    using BR              = typename LAY::BR;
-    constexpr int  N      = K + 1, NT = BR::NT, NP = BR::NPTS, PX = BR::PX, PY = BR::PY;
-    constexpr int  BX     = BR::BX, BY = BR::BY;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *const s_src = reinterpret_cast<T *>(smem_raw);
-    T *const s_dst = s_src + NP;
-    __shared__ unsigned s_ticket;
-    if (a.skip != nullptr && *a.skip != 0)
-      return;
-
-    BR br;
-    if (!brick_begin<BR, T, MODE>(br, a.g, a.s, a.dst, a.b, &s_ticket))
-      return;
-    for (int p = threadIdx.x; p < NP; p += NT)
-      s_dst[p] = T(0);
-    // SUPG with a DoF-vector velocity reads each component three times per cell: staged per brick
-    constexpr bool STAGE = SUPG && VDOF && LAY::STAGE_FIELD;
-    double *const  s_f   = reinterpret_cast<double *>(s_dst + NP);
-    if constexpr (STAGE)
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        brick_stage<BR, double, false>(br, a.vfield[d], false, s_f + d * NP);
-    brick_stage(br, a.src, a.mask_src != 0, s_src);
-
-    const int  tx = threadIdx.x % BX, ty = (threadIdx.x / BX) % BY, tz = threadIdx.x / (BX * BY);
-    const int  cx = br.c0[0] + tx, cy = br.c0[1] + ty, cz = br.c0[2] + tz;
-    const bool valid = cx < a.g.m[0] && cy < a.g.m[1] && cz < a.g.m[2];
-    const int  base = (K * tz) * PY * PX + (K * ty) * PX + K * tx;
-
-    const T *tb  = adv_table<T>(K);
-    const T *tB  = tb, *tD = tb + N * N, *tqp = tb + 2 * N * N, *tw3 = tb + 2 * N * N + N;
-    // velocity component d of a DoF-vector field at the cell's Gauss points
-    auto field = [&](int d, T *vq) {
-      if constexpr (STAGE)
-        field_at_points_staged<T, N, PX, PY>(s_f + d * NP, base, tB, vq);
-      else
-        field_at_points<T, N>(a.vfield[d], a.g, cx, cy, cz, tB, vq);
+    static constexpr int  N = K + 1, N3 = N * N * N;
+    static constexpr bool NODES = false;
+    const AdvArgs<T, N> &a;
+    struct Cell
+    {
+      int c[3];
     };
-    T uq[N * N * N], R[N * N * N];
-    if (valid)
-      {
+    __device__ __forceinline__ Cell
+    load(bool, int cx, int cy, int cz) const
+    {
+      // a lane outside the mesh reads the field of the nearest cell
+      return Cell{{min(cx, a.g.m[0] - 1), min(cy, a.g.m[1] - 1), cz}};
+    }
+    // component d of a DoF-vector velocity at the cell's Gauss points (read plainly, :461-466)
+    __device__ __forceinline__ void
+    field(int d, const Cell &c, T *v) const
+    {
+      const double *f = a.vfield[d] + ((long long)(K * c.c[0]) + (long long)a.g.n[0] * ((long long)(K * c.c[1]) + (long long)a.g.n[1] * (K * c.c[2])));
+      const int sy = a.g.n[0], sz = a.g.n[0] * a.g.n[1];
 #pragma unroll
-        for (int l = 0; l < N; ++l)
+      for (int l = 0; l < N; ++l)
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+        for (int j = 0; j < N; ++j)
 #pragma unroll
-            for (int i = 0; i < N; ++i)
-              uq[(l * N + j) * N + i] = s_src[base + l * PY * PX + j * PX + i];
-        sweep<T, N, 0, false>(uq, tB);
-        sweep<T, N, 1, false>(uq, tB);
-        sweep<T, N, 2, false>(uq, tB);
-        // cell origin and the velocity there
-        const T x0 = a.origin[0] + a.h[0] * cx, y0 = a.origin[1] + a.h[1] * cy, z0 = a.origin[2] + a.h[2] * cz;
-#pragma unroll
-        for (int q = 0; q < N * N * N; ++q)
-          R[q] = a.pm[q] * uq[q];
+          for (int i = 0; i < N; ++i)
+            v[(l * N + j) * N + i] = (T)__ldg(f + (j * sy + l * sz + i));
+      gp_interpolate<T, N, 0>(v, a.B);
+      gp_interpolate<T, N, 1>(v, a.B);
+      gp_interpolate<T, N, 2>(v, a.B);
+    }
+    __device__ __forceinline__ T
+    tau_of(T speed2) const
+    {
+      if (a.supg_coef >= T(0))
+        return a.supg_coef * a.cell_size;
+      const T vmax = sqrt(speed2);
+      return (vmax >= T(1e-6) ? T(1) / vmax : T(0)) * a.cell_size;
+    }
+    template <bool DOT>
+    __device__ __forceinline__ double
+    apply(T *u, const Cell &c) const
+    {
+      T    S[N3], s[SUPG ? N3 : 1];
+      const bool dif = a.dif != 0;
+      gp_interpolate<T, N, 0>(u, a.B);
+      gp_interpolate<T, N, 1>(u, a.B);
+      gp_interpolate<T, N, 2>(u, a.B);
+      if constexpr (VDOF)
         {
-          const T th_adv = a.th_adv, th_dif = a.th_dif;
+          // FP32 keeps the three components for the SUPG test (81 registers); FP64 interpolates them
+          // twice, with |v|^2 summed over the first pass
+          constexpr bool KEEP = SUPG && sizeof(T) == 4 && K <= 2;
+          T              v[KEEP ? 3 : 1][N3], n2[SUPG && !KEEP ? N3 : 1];
+          auto           at = [&](int d) { return KEEP ? d : 0; };
 #define MPDG_ADV_DIR(d)                                                                                         \
   {                                                                                                             \
-    const T vd0 = a.vel[d] + a.vel[3 + 3 * d] * x0 + a.vel[4 + 3 * d] * y0 + a.vel[5 + 3 * d] * z0;            \
-    if constexpr (VDOF)                                                                                         \
-      {                                                                                                         \
-        T vq[N * N * N];                                                                                        \
-        field(d, vq);                                                                                           \
-        adv_direction<T, N, d>(uq, R, tD, a.pa[d], a.pb[d], a.pd[d], vd0, th_dif != T(0), vq);                  \
-      }                                                                                                         \
-    else                                                                                                        \
-      adv_direction<T, N, d>(uq, R, tD, a.pa[d], a.pb[d], a.pd[d], vd0, th_dif != T(0));                       \
+    T *vd = v[at(d)];                                                                                          \
+    field(d, c, vd);                                                                                           \
+    adv_direction<T, N, d, d == 0, SUPG>(u, S, s, a.D[d], a.L[d], a.E[d], a.mass, dif, [&](int q) { return vd[q]; });  \
+    if constexpr (SUPG && !KEEP)                                                                                \
+      _Pragma("unroll") for (int q = 0; q < N3; ++q) n2[q] = d == 0 ? vd[q] * vd[q] : fma(vd[q], vd[q], n2[q]); \
   }
-          if constexpr (SUPG && VDOF)
-            {
-              // SUPG with a DoF-vector velocity: one component at the Gauss points at a time (four
-              // cell arrays live: u_q, R, the strong residual and the component).  Pass 1: the
-              // advection terms and |v|^2 at the points (kept in the residual's array) for tau_c
-              // (advection_diffusion_operator.cpp:510-520); pass 2: the strong residual; pass 3 its test
-              // with tau_c v.grad phi.
-              T sres[N * N * N], vq[N * N * N];
-#pragma unroll
-              for (int q = 0; q < N * N * N; ++q)
-                sres[q] = T(0);
-#pragma unroll
-              for (int d = 0; d < 3; ++d)
-                {
-                  field(d, vq);
-                  if (d == 0)
-                    adv_direction<T, N, 0>(uq, R, tD, a.pa[0], a.pb[0], a.pd[0], T(0), th_dif != T(0), vq);
-                  else if (d == 1)
-                    adv_direction<T, N, 1>(uq, R, tD, a.pa[1], a.pb[1], a.pd[1], T(0), th_dif != T(0), vq);
-                  else
-                    adv_direction<T, N, 2>(uq, R, tD, a.pa[2], a.pb[2], a.pd[2], T(0), th_dif != T(0), vq);
-#pragma unroll
-                  for (int q = 0; q < N * N * N; ++q)
-                    sres[q] = fma(vq[q], vq[q], sres[q]);
-                }
-              T tau = a.supg_coef;
-              if (tau < T(0))
-                {
-                  T vmax = T(0);
-#pragma unroll
-                  for (int q = 0; q < N * N * N; ++q)
-                    vmax = fmax(vmax, sqrt(sres[q]));
-                  tau = vmax >= T(1e-6) ? T(1) / vmax : T(0);
-                }
-              tau *= a.cell_size;
-#pragma unroll
-              for (int q = 0; q < N * N * N; ++q)
-                sres[q] = a.inv_dt * uq[q];
-              const T ih[3] = {T(1) / a.h[0], T(1) / a.h[1], T(1) / a.h[2]};
-              const T z     = T(0);
-              field(0, vq);
-              supg_residual<T, N, 0>(uq, sres, tD, tqp, ih[0], z, z, z, z, th_adv, th_dif, vq);
-              field(1, vq);
-              supg_residual<T, N, 1>(uq, sres, tD, tqp, ih[1], z, z, z, z, th_adv, th_dif, vq);
-              field(2, vq);
-              supg_residual<T, N, 2>(uq, sres, tD, tqp, ih[2], z, z, z, z, th_adv, th_dif, vq);
-              const T td = tau * a.det;
-              field(0, vq);
-              supg_test<T, N, 0>(sres, R, tD, tqp, tw3, td * ih[0], z, z, z, z, vq);
-              field(1, vq);
-              supg_test<T, N, 1>(sres, R, tD, tqp, tw3, td * ih[1], z, z, z, z, vq);
-              field(2, vq);
-              supg_test<T, N, 2>(sres, R, tD, tqp, tw3, td * ih[2], z, z, z, z, vq);
-            }
-          else
-            {
-              MPDG_ADV_DIR(0)
-              MPDG_ADV_DIR(1)
-              MPDG_ADV_DIR(2)
-            }
+          MPDG_ADV_DIR(0)
+          MPDG_ADV_DIR(1)
+          MPDG_ADV_DIR(2)
 #undef MPDG_ADV_DIR
-          if constexpr (SUPG && !VDOF)
+          if constexpr (SUPG)
             {
-              const T tau = supg_tau<T, N>(a.vel, a.h, tqp, x0, y0, z0, a.supg_coef, a.cell_size);
-              T       sres[N * N * N];
+              T most = T(0);
 #pragma unroll
-              for (int q = 0; q < N * N * N; ++q)
-                sres[q] = a.inv_dt * uq[q];
-              T vd0[3], gv[3][3], ih[3];
-#pragma unroll
-              for (int d = 0; d < 3; ++d)
+              for (int q = 0; q < N3; ++q)
                 {
-                  ih[d]  = T(1) / a.h[d];
-                  vd0[d] = a.vel[d] + a.vel[3 + 3 * d] * x0 + a.vel[4 + 3 * d] * y0 + a.vel[5 + 3 * d] * z0;
-#pragma unroll
-                  for (int e = 0; e < 3; ++e)
-                    gv[d][e] = a.vel[3 + 3 * d + e] * a.h[e];
+                  if constexpr (KEEP)
+                    most = fmax(most, fma(v[2][q], v[2][q], fma(v[1][q], v[1][q], v[0][q] * v[0][q])));
+                  else
+                    most = fmax(most, n2[q]);
                 }
-              supg_residual<T, N, 0>(uq, sres, tD, tqp, ih[0], vd0[0], gv[0][0], gv[0][1], gv[0][2], th_adv, th_dif);
-              supg_residual<T, N, 1>(uq, sres, tD, tqp, ih[1], vd0[1], gv[1][0], gv[1][1], gv[1][2], th_adv, th_dif);
-              supg_residual<T, N, 2>(uq, sres, tD, tqp, ih[2], vd0[2], gv[2][0], gv[2][1], gv[2][2], th_adv, th_dif);
-              const T td = tau * a.det;
-              supg_test<T, N, 0>(sres, R, tD, tqp, tw3, td * ih[0], vd0[0], gv[0][0], gv[0][1], gv[0][2]);
-              supg_test<T, N, 1>(sres, R, tD, tqp, tw3, td * ih[1], vd0[1], gv[1][0], gv[1][1], gv[1][2]);
-              supg_test<T, N, 2>(sres, R, tD, tqp, tw3, td * ih[2], vd0[2], gv[2][0], gv[2][1], gv[2][2]);
+              const T tau = tau_of(most);
+#pragma unroll
+              for (int q = 0; q < N3; ++q)
+                s[q] *= tau;
+#define MPDG_ADV_TEST(d)                                                                                        \
+  {                                                                                                             \
+    T *vd = v[at(d)];                                                                                          \
+    if constexpr (!KEEP)                                                                                        \
+      field(d, c, vd);                                                                                         \
+    gp_divergence<T, N, d>(S, a.P[d], [&](int q) { return vd[q] * s[q]; });                                        \
+  }
+              MPDG_ADV_TEST(2)
+              MPDG_ADV_TEST(1)
+              MPDG_ADV_TEST(0)
+#undef MPDG_ADV_TEST
             }
         }
-        sweep<T, N, 2, true>(R, tB);
-        sweep<T, N, 1, true>(R, tB);
-        sweep<T, N, 0, true>(R, tB);
-        // cells sharing a lattice point add into the brick accumulator concurrently
+      else
+        {
+          T v0[3];
 #pragma unroll
-        for (int l = 0; l < N; ++l)
+          for (int d = 0; d < 3; ++d)
+            {
+              double t = a.vel[d];
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+              for (int e = 0; e < 3; ++e)
+                t = fma(a.vel[3 + 3 * d + e], fma(a.h[e], (double)c.c[e], a.origin[e]), t);
+              v0[d] = (T)t;
+            }
+          auto velocity = [&](int d, int q) {
+            return ((v0[d] + a.voff[d][2][q / (N * N)]) + a.voff[d][1][q / N % N]) + a.voff[d][0][q % N];
+          };
+          adv_direction<T, N, 0, true, SUPG>(u, S, s, a.D[0], a.L[0], a.E[0], a.mass, dif, [&](int q) { return velocity(0, q); });
+          adv_direction<T, N, 1, false, SUPG>(u, S, s, a.D[1], a.L[1], a.E[1], a.mass, dif, [&](int q) { return velocity(1, q); });
+          adv_direction<T, N, 2, false, SUPG>(u, S, s, a.D[2], a.L[2], a.E[2], a.mass, dif, [&](int q) { return velocity(2, q); });
+          if constexpr (SUPG)
+            {
+              T most = T(0);
+              if (a.supg_coef < T(0))
 #pragma unroll
-            for (int i = 0; i < N; ++i)
-              atomicAdd(s_dst + (base + l * PY * PX + j * PX + i), R[(l * N + j) * N + i]);
-      }
-    __syncthreads();
-    brick_end<BR, T, MODE>(br, a.g, a.s, s_dst, a.dst, a.b);
+                for (int q = 0; q < N3; ++q)
+                  {
+                    const T v1 = velocity(0, q), v2 = velocity(1, q), v3 = velocity(2, q);
+                    most = fmax(most, fma(v3, v3, fma(v2, v2, v1 * v1)));
+                  }
+              const T tau = tau_of(most);
+#pragma unroll
+              for (int q = 0; q < N3; ++q)
+                s[q] *= tau;
+              gp_divergence<T, N, 0>(S, a.P[0], [&](int q) { return velocity(0, q) * s[q]; });
+              gp_divergence<T, N, 1>(S, a.P[1], [&](int q) { return velocity(1, q) * s[q]; });
+              gp_divergence<T, N, 2>(S, a.P[2], [&](int q) { return velocity(2, q) * s[q]; });
+            }
+        }
+      gp_test<T, N, 2>(S, a.Bt[2]);
+      gp_test<T, N, 1>(S, a.Bt[1]);
+      gp_test<T, N, 0>(S, a.Bt[0]);
+#pragma unroll
+      for (int q = 0; q < N3; ++q)
+        u[q] = S[q];
+      return 0.0;
+    }
+  };
+
+#ifndef MPDG_ADV_MINB
+#define MPDG_ADV_MINB 0
+#endif
+  // CTAs (of 128 threads) per SM the register allocation is held to
+  template <int K, typename T, bool SUPG, bool VDOF>
+  struct AdvMinBlocks
+  {
+    static constexpr bool f64 = sizeof(T) == 8;
+    static constexpr int  value = MPDG_ADV_MINB ? MPDG_ADV_MINB :
+                                 K == 1 ? (SUPG ? (f64 ? 3 : 5) : 5) :
+                                 K == 2 ? (SUPG && VDOF ? 2 : SUPG ? (f64 ? 2 : 4) : VDOF ? (f64 ? 2 : 3) : (f64 ? 3 : 5)) : 2;
+  };
+
+  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF>
+  __global__ void __launch_bounds__(MARCH_NT, AdvMinBlocks<K, T, SUPG, VDOF>::value)
+  adv_apply_kernel(const __grid_constant__ AdvArgs<T, K + 1> a)
+  {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned                        s_ticket;
+    __shared__ __align__(8) unsigned long long s_bars[2];
+    if (a.skip != nullptr && *a.skip != 0)
+      return;
+    AdvCellOp<K, T, SUPG, VDOF> op{a};
+    march_body<K, T, MODE, AdvCellOp<K, T, SUPG, VDOF>, false, true>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
+                                                                     reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
   }
 
-  // ------------------------------------------------------------------------------------------
+  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF>
   static cudaError_t
-  upload_adv_tables()
+  launch_adv_kernel(AdvArgs<T, K + 1> &a, cudaStream_t stream)
   {
-    static std::mutex           mtx;
-    static std::set<int>        done;
-    int                         dev = 0;
-    cudaError_t                 e   = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
+    auto                                   kern = adv_apply_kernel<K, T, MODE, SUPG, VDOF>;
+    static std::atomic<unsigned long long> devices{0};
+    constexpr size_t                       bytes = MarchLayout<K, T>::bytes;
+    if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
       return e;
-    std::lock_guard<std::mutex> lock(mtx);
-    if (done.count(dev))
-      return cudaSuccess;
-    double hd[ADV_KMAX + 1][ADV_TAB] = {};
-    float  hf[ADV_KMAX + 1][ADV_TAB] = {};
-    for (int K = 1; K <= ADV_KMAX; ++K)
-      {
-        const Tables1D &t = tables(K);
-        const int       n = t.n;
-        int             o = 0;
-        for (int i = 0; i < n * n; ++i)
-          hd[K][o++] = t.B[i];
-        for (int i = 0; i < n * n; ++i)
-          hd[K][o++] = t.Dq[i];
-        for (int i = 0; i < n; ++i)
-          hd[K][o++] = t.qp[i];
-        for (int qz = 0; qz < n; ++qz)
-          for (int qy = 0; qy < n; ++qy)
-            for (int qx = 0; qx < n; ++qx)
-              hd[K][o++] = t.qw[qx] * t.qw[qy] * t.qw[qz];
-        for (int i = 0; i < o; ++i)
-          hf[K][i] = (float)hd[K][i];
-      }
-    if ((e = cudaMemcpyToSymbol(c_adv_d, hd, sizeof(hd))) != cudaSuccess)
-      return e;
-    if ((e = cudaMemcpyToSymbol(c_adv_f, hf, sizeof(hf))) != cudaSuccess)
-      return e;
-    // the copies ran on the legacy stream: complete them before kernels on other streams read the tables
-    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
-      return e;
-    done.insert(dev);
-    return cudaSuccess;
+    const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, AdvMinBlocks<K, T, SUPG, VDOF>::value);
+    kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
+    return cudaGetLastError();
   }
 
   template <int K, typename T, OutMode MODE>
@@ -588,68 +382,60 @@ namespace mpdg
   launch_adv(const AdvLaunch<T> &h, cudaStream_t stream)
   {
     constexpr int   N = K + 1;
-    using LAY         = AdvLayout<K, T>;
-    AdvArgs<T, N> a;
-    cudaError_t   ue = upload_adv_tables();
-    if (ue != cudaSuccess)
-      return ue;
-    a.det = (T)(h.p.h[0] * h.p.h[1] * h.p.h[2]);
-    a.g      = h.grid;
-    a.s      = h.sync;
-    a.inv_dt = (T)(h.scale * h.p.inv_dt);
-    a.th_adv = (T)(h.scale * h.p.theta_adv);
-    a.th_dif = (T)(h.scale * h.p.theta_dif);
-    for (int i = 0; i < 12; ++i)
-      a.vel[i] = (T)h.p.vel[i];
-    for (int d = 0; d < 3; ++d)
-      {
-        a.origin[d] = (T)h.p.origin[d];
-        a.h[d]      = (T)h.p.h[d];
-      }
+    AdvArgs<T, N>   a{};
+    const Tables1D &t = tables(K);
+    a.g        = h.grid;
+    a.s        = h.sync;
     a.src      = h.src;
     a.dst      = h.dst;
     a.b        = h.b;
     a.mask_src = h.mask_src;
     a.skip     = h.skip;
+    const double ta = h.scale * h.p.theta_adv, td = h.scale * h.p.theta_dif, ti = h.scale * h.p.inv_dt;
+    const double det = h.p.h[0] * h.p.h[1] * h.p.h[2];
+    a.dif            = td != 0.0;
+    double dwd[N * N], dd[N * N]; // W^-1 D^T W D, D D
+    for (int q = 0; q < N; ++q)
+      for (int r = 0; r < N; ++r)
+        {
+          a.B[q * N + r]  = (T)t.B[q * N + r];
+          dwd[q * N + r] = dd[q * N + r] = 0.0;
+          for (int k = 0; k < N; ++k)
+            {
+              dwd[q * N + r] += t.Dq[k * N + q] * t.qw[k] * t.Dq[k * N + r] / t.qw[q];
+              dd[q * N + r] += t.Dq[q * N + k] * t.Dq[k * N + r];
+            }
+          for (int d = 0; d < 3; ++d)
+            {
+              a.Bt[d][r * N + q] = (T)((d == 2 ? det : 1.0) * t.qw[q] * t.B[q * N + r]);
+              a.P[d][q * N + r]  = (T)(t.Dq[r * N + q] * t.qw[r] / t.qw[q] / h.p.h[d]);
+            }
+        }
+    for (int d = 0; d < 3; ++d)
+      {
+        const double hd = h.p.h[d];
+        gp_on_differences<T, N>(t.Dq, ta / hd, a.D[d]);
+        gp_on_differences<T, N>(dwd, td / (hd * hd), a.L[d]);
+        gp_on_differences<T, N>(dd, td / (hd * hd), a.E[d]);
+      }
+    a.mass = (T)ti;
+    for (int d = 0; d < 3; ++d)
+      {
+        a.vfield[d] = h.p.vfield[d];
+        a.origin[d] = h.p.origin[d];
+        a.h[d]      = h.p.h[d];
+        for (int e = 0; e < 3; ++e)
+          for (int q = 0; q < N; ++q)
+            a.voff[d][e][q] = (T)(h.p.vel[3 + 3 * d + e] * h.p.h[e] * t.qp[q]);
+      }
+    for (int i = 0; i < 12; ++i)
+      a.vel[i] = h.p.vel[i];
     a.supg_coef = (T)h.p.supg_coef;
     a.cell_size = (T)(std::sqrt(h.p.h[0] * h.p.h[0] + h.p.h[1] * h.p.h[1] + h.p.h[2] * h.p.h[2]) / std::sqrt(3.0));
-    for (int d = 0; d < 3; ++d)
-      a.vfield[d] = h.p.vfield[d];
-    {
-      // cell-independent point factors (see AdvArgs), in double, rounded once
-      const Tables1D &t   = tables(K);
-      const double    det = h.p.h[0] * h.p.h[1] * h.p.h[2];
-      const double    ta = h.scale * h.p.theta_adv, td = h.scale * h.p.theta_dif, ti = h.scale * h.p.inv_dt;
-      for (int qz = 0; qz < N; ++qz)
-        for (int qy = 0; qy < N; ++qy)
-          for (int qx = 0; qx < N; ++qx)
-            {
-              const int    q  = (qz * N + qy) * N + qx;
-              const double w3 = t.qw[qx] * t.qw[qy] * t.qw[qz];
-              a.pm[q]         = (T)(det * ti * w3);
-              for (int d = 0; d < 3; ++d)
-                {
-                  const double pa = ta * det / h.p.h[d] * w3;
-                  const double gv = h.p.vel[3 + 3 * d] * h.p.h[0] * t.qp[qx] + h.p.vel[4 + 3 * d] * h.p.h[1] * t.qp[qy] +
-                                    h.p.vel[5 + 3 * d] * h.p.h[2] * t.qp[qz];
-                  a.pa[d][q] = (T)pa;
-                  a.pb[d][q] = (T)(pa * gv);
-                  a.pd[d][q] = (T)(td * det / (h.p.h[d] * h.p.h[d]) * w3);
-                }
-            }
-    }
     const bool vdof = h.p.vfield[0] != nullptr;
-    auto kern = h.p.supg ? (vdof ? adv_apply_kernel<K, T, MODE, true, true> : adv_apply_kernel<K, T, MODE, true>)
-                         : (vdof ? adv_apply_kernel<K, T, MODE, false, true> : adv_apply_kernel<K, T, MODE, false>);
-    static std::atomic<unsigned long long> devices{0}, devices_supg{0}, devices_vdof{0}, devices_sv{0};
-    const size_t bytes = h.p.supg && vdof && LAY::STAGE_FIELD ? LAY::bytes_staged : LAY::bytes;
-    if (cudaError_t e = ensure_smem(kern, bytes,
-                                    h.p.supg ? (vdof ? devices_sv : devices_supg) : (vdof ? devices_vdof : devices));
-        e != cudaSuccess)
-      return e;
-    const unsigned nbricks = (unsigned)h.grid.nbr[0] * h.grid.nbr[1] * h.grid.nbr[2];
-    kern<<<nbricks, LAY::BR::NT, bytes, stream>>>(a);
-    return cudaGetLastError();
+    if (h.p.supg)
+      return vdof ? launch_adv_kernel<K, T, MODE, true, true>(a, stream) : launch_adv_kernel<K, T, MODE, true, false>(a, stream);
+    return vdof ? launch_adv_kernel<K, T, MODE, false, true>(a, stream) : launch_adv_kernel<K, T, MODE, false, false>(a, stream);
   }
 
   template <int K, typename T>
@@ -681,26 +467,19 @@ namespace mpdg
   void
   adv_brick_shape(int K, int shape[3])
   {
-    if (K == 1)
-      {
-        shape[0] = AdvLayout<1, T>::BX;
-        shape[1] = AdvLayout<1, T>::BY;
-        shape[2] = AdvLayout<1, T>::BZ;
-      }
-    else if (K == 2)
-      {
-        shape[0] = AdvLayout<2, T>::BX;
-        shape[1] = AdvLayout<2, T>::BY;
-        shape[2] = AdvLayout<2, T>::BZ;
-      }
-    else
-      {
-        shape[0] = AdvLayout<3, T>::BX;
-        shape[1] = AdvLayout<3, T>::BY;
-        shape[2] = AdvLayout<3, T>::BZ;
-      }
+    shape[0] = MARCH_BX;
+    shape[1] = MARCH_BY;
+    shape[2] = K == 1 ? MarchShape<1, T>::BZ : (K == 2 ? MarchShape<2, T>::BZ : MarchShape<3, T>::BZ);
   }
 
+  long long
+  adv_flags(int K, const int m[3])
+  {
+    int sd[3], sf[3];
+    adv_brick_shape<double>(K, sd);
+    adv_brick_shape<float>(K, sf);
+    return std::max(march_flags(m, sd[2]), march_flags(m, sf[2]));
+  }
 
   // ---- diagonal in closed form (MatrixFreeTools::compute_diagonal of the tangent).
   // With phi_i = phi_a(x) phi_b(y) phi_c(z) and an affine velocity, every term of

@@ -1150,19 +1150,8 @@ mpdg_op_create(const mpdg_mesh_desc *mesh, const mpdg_op_params *params, mpdg_op
                             (long long)op->nbr32[0] * op->nbr32[1] * op->nbr32[2]);
   if (op->kind == MPDG_HEAT)
     nbrk = std::max(nbrk, heat_flags(op->degree, op->m, mesh->dirichlet_mask == nullptr));
-  if (op->kind == MPDG_HEAT && op->degree <= 3)
-    for (int prec = 0; prec < 2; ++prec)
-      {
-        int sh[3];
-        if (prec == 0)
-          adv_brick_shape<double>(op->degree, sh);
-        else
-          adv_brick_shape<float>(op->degree, sh);
-        long long nb = 1;
-        for (int d = 0; d < 3; ++d)
-          nb *= (op->m[d] + sh[d] - 1) / sh[d];
-        nbrk = std::max(nbrk, nb);
-      }
+  if (op->degree <= 3)
+    nbrk = std::max(nbrk, adv_flags(op->degree, op->m));
   auto            clean = [&](int code, const std::string &msg) {
     mpdg_op_destroy(op);
     return fail(code, msg);

@@ -306,7 +306,8 @@ namespace mpdg
   template <int K, typename T>
   struct HeatCellOp
   {
-    static constexpr int N = K + 1, NE = (N + 1) / 2, NO = N / 2;
+    static constexpr int  N = K + 1, NE = (N + 1) / 2, NO = N / 2;
+    static constexpr bool NODES = false;
     const HeatArgs<T, N> &a;
     // conductivity of the cell (unscaled)
     __device__ __forceinline__ T
@@ -610,8 +611,7 @@ namespace mpdg
       if (h.grid.cmask == nullptr && h.march)
         {
           using ML = MarchLayout<K, T>;
-          a.g.bz = march_plan(a.g.m, MarchShape<K, T>::BZ, 148 * MarchMinBlocks<K, T>::value, &a.g.nbr[2]);
-          const unsigned nbricks = (unsigned)a.g.nbr[0] * a.g.nbr[1] * a.g.nbr[2];
+          const unsigned nbricks = march_grid(a.g, MarchShape<K, T>::BZ, MarchMinBlocks<K, T>::value);
           static std::atomic<unsigned long long> dev_plain{0}, dev_dot{0};
           if constexpr (MODE == OutMode::Set)
             if (h.dot.part != nullptr)

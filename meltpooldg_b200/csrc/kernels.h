@@ -196,6 +196,8 @@ namespace mpdg
 
   template <typename T>
   void adv_brick_shape(int K, int shape[3]);
+  // init flags that an advection-form apply of this mesh may use, in either precision
+  long long adv_flags(int K, const int m[3]);
 
   // ---- vectors and reductions (double accumulation for every vector type)
   constexpr int RED_BLOCKS  = 592; // 4 x 148 SMs

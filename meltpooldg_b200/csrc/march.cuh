@@ -77,6 +77,17 @@ namespace mpdg
     return bz;
   }
 
+  // The column counts and the segment length of a launch on 148 SMs with per_sm resident CTAs; returns
+  // the number of CTAs.
+  inline unsigned
+  march_grid(GridDesc &g, int bz_full, int per_sm)
+  {
+    g.nbr[0] = (g.m[0] + MARCH_BX - 1) / MARCH_BX;
+    g.nbr[1] = (g.m[1] + MARCH_BY - 1) / MARCH_BY;
+    g.bz     = march_plan(g.m, bz_full, 148 * per_sm, &g.nbr[2]);
+    return (unsigned)g.nbr[0] * g.nbr[1] * g.nbr[2];
+  }
+
   // flags / dot partials an operator must hold for the segments of any of its marching applies
   inline long long
   march_flags(const int m[3], int bz_full)
@@ -303,9 +314,19 @@ namespace mpdg
       row(r, true);
   }
 
+  // The cell's nodal values in the ring, for operators that read them several times instead of holding them:
+  // row (l, j) of the cell, N values.  Constrained values are zeroed in the ring before.
+  template <int K, typename T>
+  struct MarchNodes
+  {
+    const T *row[(K + 1) * (K + 1)];
+  };
+
   // The marching body.  Cell operator: op.apply<DOT>(u, op.load(valid, cx, cy, cz)) in place on (K+1)^3 values.
   // With DOT the cell operator returns the cell's form src_c^T A src_c and the sum over the segment goes
   // to the fused dot product (release_ticket_dot).
+  // An operator with Op::NODES instead has op.apply(u, nodes, op.load(...)): it reads its input through
+  // MarchNodes and only writes u.
   // MASKABLE: the operator may carry per-DoF constraint flags (GridDesc::cmask) besides the faces.
   template <int K, typename T, OutMode MODE, class Op, bool DOT = false, bool MASKABLE = false>
   __device__ __forceinline__ void
@@ -378,58 +399,89 @@ namespace mpdg
           atomicExch(s.error, ERR_FLAG_WAIT);
         const bool last_layer = lz == nlayers - 1;
         const bool cL0 = br.con_lo[2] && cz == 0, cLK = br.con_hi[2] && cz == g.m[2] - 1;
-        T          u[N * N * N];
+        T                u[N * N * N];
+        MarchNodes<K, T> nodes;
 #pragma unroll
         for (int l = 0; l < N; ++l)
           {
             int sl = slot0 + l;
             if (sl >= NRING)
               sl -= NRING;
-            const T *pl = ring + sl * LAY::PLANE + (K * warp) * PITCH + K * lane;
-            const int e = base + wbase + br.sz * (K * lz + l);
+            const T  *pl = ring + sl * LAY::PLANE + (K * warp) * PITCH + K * lane;
+            const int e  = base + wbase + br.sz * (K * lz + l);
 #pragma unroll
             for (int j = 0; j < N; ++j)
-              {
-                const T *row = pl + j * PITCH + ((e + j * br.sy) & (G - 1));
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-                  u[(l * N + j) * N + i] = row[i];
-              }
+              nodes.row[l * N + j] = pl + j * PITCH + ((e + j * br.sy) & (G - 1));
           }
         slot0 += K;
         if (slot0 >= NRING)
           slot0 -= NRING;
-        if (do_mask)
+        if constexpr (Op::NODES)
+          {
+            // constrained entry (i, j, l) of the cell: Dirichlet planes, per-DoF flags
+            auto constrained = [&](int i, int j, int l) {
+              bool con = (l == 0 && cL0) || (l == K && cLK) || (j == 0 && cJ0) || (j == K && cJK) || (i == 0 && cI0) ||
+                         (i == K && cIK);
+              if constexpr (MASKABLE)
+                con = con || (g.cmask != nullptr && g.cmask[wbase + K * lane + i + j * br.sy + br.sz * (K * lz + l)]);
+              return con;
+            };
+            const bool masked = do_mask || (MASKABLE && mask_src && g.cmask != nullptr); // the same for the whole CTA
+            if (masked)
+              {
+                // every thread zeroes its cell's constrained values (cells that share one write the same)
+                if (vxy)
+#pragma unroll
+                  for (int l = 0; l < N; ++l)
+#pragma unroll
+                    for (int j = 0; j < N; ++j)
+#pragma unroll
+                      for (int i = 0; i < N; ++i)
+                        if (constrained(i, j, l))
+                          const_cast<T *>(nodes.row[l * N + j])[i] = T(0);
+                __syncthreads();
+              }
+            op.apply(u, nodes, pre);
+          }
+        else
           {
 #pragma unroll
-            for (int l = 0; l < N; ++l)
+            for (int r = 0; r < N * N; ++r)
 #pragma unroll
-              for (int j = 0; j < N; ++j)
+              for (int i = 0; i < N; ++i)
+                u[r * N + i] = nodes.row[r][i];
+            if (do_mask)
+              {
+#pragma unroll
+                for (int l = 0; l < N; ++l)
+#pragma unroll
+                  for (int j = 0; j < N; ++j)
+                    {
+                      const bool cr = (l == 0 && cL0) || (l == K && cLK) || (j == 0 && cJ0) || (j == K && cJK);
+#pragma unroll
+                      for (int i = 0; i < N; ++i)
+                        if (cr || (i == 0 && cI0) || (i == K && cIK))
+                          u[(l * N + j) * N + i] = T(0);
+                    }
+              }
+            if constexpr (MASKABLE)
+              if (g.cmask != nullptr && mask_src && vxy)
                 {
-                  const bool cr = (l == 0 && cL0) || (l == K && cLK) || (j == 0 && cJ0) || (j == K && cJK);
+                  const uint8_t *cm = g.cmask + (wbase + K * lane + br.sz * (K * lz));
 #pragma unroll
-                  for (int i = 0; i < N; ++i)
-                    if (cr || (i == 0 && cI0) || (i == K && cIK))
-                      u[(l * N + j) * N + i] = T(0);
+                  for (int l = 0; l < N; ++l)
+#pragma unroll
+                    for (int j = 0; j < N; ++j)
+#pragma unroll
+                      for (int i = 0; i < N; ++i)
+                        if (cm[j * br.sy + l * br.sz + i])
+                          u[(l * N + j) * N + i] = T(0);
                 }
+            if constexpr (DOT)
+              dsum += vxy ? op.template apply<true>(u, pre) : 0.0;
+            else
+              op.template apply<false>(u, pre);
           }
-        if constexpr (MASKABLE)
-          if (g.cmask != nullptr && mask_src && vxy)
-            {
-              const uint8_t *cm = g.cmask + (wbase + K * lane + br.sz * (K * lz));
-#pragma unroll
-              for (int l = 0; l < N; ++l)
-#pragma unroll
-                for (int j = 0; j < N; ++j)
-#pragma unroll
-                  for (int i = 0; i < N; ++i)
-                    if (cm[j * br.sy + l * br.sz + i])
-                      u[(l * N + j) * N + i] = T(0);
-            }
-        if constexpr (DOT)
-          dsum += vxy ? op.template apply<true>(u, pre) : 0.0;
-        else
-          op.template apply<false>(u, pre);
         // x: lane t adds lane t-1's x = K face
 #pragma unroll
         for (int q = 0; q < N * N; ++q)
@@ -486,8 +538,9 @@ namespace mpdg
                 d0[off] = con ? T(0) : v;
               else if constexpr (MODE == OutMode::Add)
                 {
+                  // a reduction without a return value: nothing waits for the old value
                   if (!con)
-                    d0[off] += v;
+                    atomicAdd(d0 + off, v);
                 }
               else
                 d0[off] = con ? bvec[cbase + off] : bvec[cbase + off] + v;
