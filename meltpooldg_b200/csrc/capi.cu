@@ -247,19 +247,6 @@ namespace
   // vector): rho c_p / dt u + rho c_p v . grad u tested with phi plus k grad u . grad phi, i.e. the
   // advection-diffusion form with 1/dt -> rho c_p / dt, theta -> rho c_p, theta eps -> k (the
   // velocity term alone for create_rhs: adv = -rho c_p, no mass, no diffusion).
-  // the lattice of a heat operator with the brick counts of the advection-form kernels
-  template <typename T>
-  GridDesc
-  heat_velocity_grid(const mpdg_op *op)
-  {
-    GridDesc g = op->grid<T>();
-    int      sh[3];
-    adv_brick_shape<T>(op->degree, sh);
-    for (int d = 0; d < 3; ++d)
-      g.nbr[d] = (op->m[d] + sh[d] - 1) / sh[d];
-    return g;
-  }
-
   AdvParams
   heat_velocity_params(const mpdg_op *op, bool rhs_term)
   {
@@ -387,11 +374,11 @@ namespace
       {
         // the projection operator M + damping K with a narrow band (normal_vector_operator.cpp:
         // 326-358, curvature_operator.cpp:337-369): the isotropic form of the point-wise kernel
-        if (mode == (int)OutMode::Set)
-          MPDG_CUDA(vec_fill<T>(dst, T(0), op->ndofs, op->stream));
-        else if (mode == (int)OutMode::BPlus && dst != b)
-          MPDG_CUDA(cudaMemcpyAsync(dst, b, sizeof(T) * op->ndofs, cudaMemcpyDeviceToDevice, op->stream));
-        MPDG_CUDA(reinit_integrate<T>(band_launch<T>(op, which, scale, src, dst, mask_src), 0, op->stream));
+        ReinitLaunch<T> r = band_launch<T>(op, which, scale, src, dst, mask_src);
+        r.out_mode        = mode;
+        r.sync            = op->sync();
+        r.b               = b;
+        MPDG_CUDA(reinit_integrate<T>(r, 0, op->stream));
         return MPDG_OK;
       }
     if (op->kind == MPDG_HEAT)
@@ -427,7 +414,7 @@ namespace
             a.mode     = mode;
             a.scale    = scale;
             a.p        = heat_velocity_params(op, false);
-            a.grid     = heat_velocity_grid<T>(op);
+            a.grid     = op->grid<T>();
             a.sync     = op->sync();
             a.src      = src;
             a.dst      = dst;
@@ -459,12 +446,11 @@ namespace
       {
         if (!op->d_normal[0] || !op->d_normal[1] || !op->d_normal[2])
           return fail(MPDG_ERR_ARG, "the reinitialisation operator needs its normal field (mpdg_op_set_reinit)");
-        // dst prepared for the atomics of the cell kernel: 0 (Set) or b (BPlus); Add adds in place
-        if (mode == (int)OutMode::Set)
-          MPDG_CUDA(vec_fill<T>(dst, T(0), op->ndofs, op->stream));
-        else if (mode == (int)OutMode::BPlus && dst != b)
-          MPDG_CUDA(cudaMemcpyAsync(dst, b, sizeof(T) * op->ndofs, cudaMemcpyDeviceToDevice, op->stream));
-        MPDG_CUDA(reinit_integrate<T>(reinit_launch<T>(op, scale, src, dst, mask_src), 0, op->stream));
+        ReinitLaunch<T> r = reinit_launch<T>(op, scale, src, dst, mask_src);
+        r.out_mode        = mode;
+        r.sync            = op->sync();
+        r.b               = b;
+        MPDG_CUDA(reinit_integrate<T>(r, 0, op->stream));
       }
     else
       {
@@ -1420,7 +1406,7 @@ mpdg_level_set_normal_rhs(mpdg_op *op, const double *psi, int normalized, double
   if (op->degree > 3)
     return fail(MPDG_ERR_UNSUPPORTED, "the level-set right-hand sides support FE_Q degree 1..3");
   // the normal's narrow band masks with the level set psi itself (normal_vector_operator.cpp:184-189)
-  MPDG_CUDA(level_set_rhs(op->grid(), op->degree, op->h, 0, normalized ? 1 : 0, 0.0, psi, nullptr, nullptr, nx, ny,
+  MPDG_CUDA(level_set_rhs(op->grid(), op->sync(), op->degree, op->h, 0, normalized ? 1 : 0, 0.0, psi, nullptr, nullptr, nx, ny,
                           nz, op->stream, op->banded() ? psi : nullptr, op->band));
   return MPDG_OK;
 }
@@ -1435,8 +1421,7 @@ mpdg_level_set_curvature_rhs(mpdg_op *op, const double *nx, const double *ny, co
     return fail(MPDG_ERR_ARG, "invalid argument to mpdg_level_set_curvature_rhs");
   if (op->degree > 3)
     return fail(MPDG_ERR_UNSUPPORTED, "the level-set right-hand sides support FE_Q degree 1..3");
-  MPDG_CUDA(vec_fill<double>(dst, 0.0, op->ndofs, op->stream));
-  MPDG_CUDA(level_set_rhs(op->grid(), op->degree, op->h, 1, 0, normal_tolerance, nx, ny, nz, dst, nullptr, nullptr,
+  MPDG_CUDA(level_set_rhs(op->grid(), op->sync(), op->degree, op->h, 1, 0, normal_tolerance, nx, ny, nz, dst, nullptr, nullptr,
                           op->stream, op->banded() ? op->d_band_ls : nullptr, op->band));
   return MPDG_OK;
 }
@@ -1822,8 +1807,10 @@ mpdg_op_create_rhs(mpdg_op *op, double *dst, const double *a, const double *b, c
       // olsson_CG_operator.cpp:197-260: dst is overwritten, constrained rows end at 0
       if (!op->d_normal[0] || !op->d_normal[1] || !op->d_normal[2])
         return fail(MPDG_ERR_ARG, "the reinitialisation operator needs its normal field (mpdg_op_set_reinit)");
-      MPDG_CUDA(vec_fill<double>(dst, 0.0, op->ndofs, op->stream));
-      MPDG_CUDA(reinit_integrate<double>(reinit_launch<double>(op, 1.0, a, dst, 0), 1, op->stream));
+      ReinitLaunch<double> r = reinit_launch<double>(op, 1.0, a, dst, 0);
+      r.out_mode             = (int)OutMode::Set;
+      r.sync                 = op->sync();
+      MPDG_CUDA(reinit_integrate<double>(r, 1, op->stream));
       return MPDG_OK;
     }
   if (op->kind == MPDG_HEAT && op->solid)
@@ -1873,7 +1860,7 @@ mpdg_op_create_rhs(mpdg_op *op, double *dst, const double *a, const double *b, c
           h.mode     = (int)OutMode::Add;
           h.scale    = 1.0;
           h.p        = heat_velocity_params(op, true);
-          h.grid     = heat_velocity_grid<double>(op);
+          h.grid     = op->grid();
           h.sync     = op->sync();
           h.src      = a;
           h.dst      = dst;

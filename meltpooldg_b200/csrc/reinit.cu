@@ -11,10 +11,11 @@
 // points while it assembles the rhs and reuses the cache in vmult; here it is evaluated from the
 // normal field at every apply (the same as long as the field does not change in between).
 //
-// One thread per cell, point-wise quadrature: at each Gauss point the value and gradient of the
-// input and the normal field come from the cell's nodal values (tensor products of the 1-D basis
-// values and derivatives), and the integrand is tested against every nodal basis function; cells
-// add into dst with atomics (dst is prepared by the host: zero, or b for b + A x).
+// The applies and right-hand sides run in the column-marching frame (march.cuh), one thread per cell, by sum
+// factorisation on the Gauss points (gausspoint.cuh).  With v = n_h at the points, D grad u = eps_t grad u +
+// c v, c = (eps_n - eps_t) (v . grad u) / |v|^2.  The tangent and the right-hand side walk the cell one plane of
+// points at a time: the three components of v, u and its derivatives at all (k+1)^3 points would not fit the
+// registers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,7 +23,9 @@
 #include <mutex>
 
 #include "brick.cuh"
+#include "gausspoint.cuh"
 #include "kernels.h"
+#include "march.cuh"
 
 namespace mpdg
 {
@@ -38,7 +41,7 @@ namespace mpdg
       const double *n[3];
       T            *dst;
       double       *diag;
-      int           mode; // 0 tangent apply, 1 rhs (src = psi_old, plain), 2 diagonal
+      int           mode; // wetting faces: 0 tangent apply, 1 rhs (src = psi_old, plain), 2 diagonal
       int           mask_src;
       const double *band_ls; // narrow band (include/meltpooldg/level_set/level_set_tools.hpp:357-368)
       T             band;
@@ -46,9 +49,10 @@ namespace mpdg
       T             Vend[2 * N], Dend[2 * N]; // basis values / derivatives at x = 0 and x = 1
     };
 
+    // Diagonal of the tangent (and of the banded isotropic form), one thread per cell, point by point
     template <int K, typename T>
     __global__ void __launch_bounds__(128)
-    reinit_kernel(const __grid_constant__ ReinitArgs<T, K + 1> a)
+    reinit_diag_kernel(const __grid_constant__ ReinitArgs<T, K + 1> a)
     {
       constexpr int   N     = K + 1, N3 = N * N * N;
       const int       m0    = a.g.m[0], m1 = a.g.m[1];
@@ -58,7 +62,7 @@ namespace mpdg
           const int cx = (int)(c % m0), cy = (int)((c / m0) % m1), cz = (int)(c / ((long long)m0 * m1));
           long long idx[N3];
           bool      con[N3];
-          T         u[N3], R[N3], ls[N3];
+          T         R[N3], ls[N3];
 #pragma unroll
           for (int l = 0; l < N; ++l)
 #pragma unroll
@@ -71,7 +75,6 @@ namespace mpdg
                   const long long id = (long long)I + (long long)a.g.n[0] * ((long long)J + (long long)a.g.n[1] * L);
                   idx[q]             = id;
                   con[q]             = is_constrained(a.g, I, J, L, id);
-                  u[q]               = (a.mode == 2 || (a.mask_src && con[q])) ? T(0) : a.src[id];
                   R[q]               = T(0);
                   ls[q]              = a.band_ls ? (T)a.band_ls[id] : T(0); // read plainly
                 }
@@ -79,9 +82,8 @@ namespace mpdg
             for (int qy = 0; qy < N; ++qy)
               for (int qx = 0; qx < N; ++qx)
                 {
-                  // value and gradient of u and the normal field at the Gauss point
-                  // (the isotropic form, eps_n == eps_t, has no normal field: n == nullptr)
-                  T uv = T(0), g[3] = {T(0), T(0), T(0)}, nv[3] = {T(0), T(0), T(0)}, lq = T(0);
+                  // the normal field (none in the isotropic form) and the level set at the Gauss point
+                  T          nv[3] = {T(0), T(0), T(0)}, lq = T(0);
                   const bool has_n = a.n[0] != nullptr;
 #pragma unroll
                   for (int l = 0; l < N; ++l)
@@ -91,21 +93,13 @@ namespace mpdg
                       for (int i = 0; i < N; ++i)
                         {
                           const int q   = (l * N + j) * N + i;
-                          const T   bx = a.B[qx * N + i], by = a.B[qy * N + j], bz = a.B[qz * N + l];
-                          const T   phi = bx * by * bz;
-                          uv += phi * u[q];
+                          const T   phi = a.B[qx * N + i] * a.B[qy * N + j] * a.B[qz * N + l];
                           lq += phi * ls[q];
-                          g[0] += a.G[qx * N + i] * by * bz * u[q];
-                          g[1] += bx * a.G[qy * N + j] * bz * u[q];
-                          g[2] += bx * by * a.G[qz * N + l] * u[q];
                           if (has_n)
 #pragma unroll
                             for (int d = 0; d < 3; ++d)
                               nv[d] += phi * (T)a.n[d][idx[q]];
                         }
-#pragma unroll
-                  for (int d = 0; d < 3; ++d)
-                    g[d] *= a.ih[d];
                   if (has_n)
                     {
                       const T nn  = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
@@ -116,44 +110,7 @@ namespace mpdg
                     }
                   // narrow band: the point contributes only where |level set| < band
                   const T jw = (a.band_ls && !(fabs(lq) < a.band)) ? T(0) : a.det * a.w[qx] * a.w[qy] * a.w[qz];
-                  if (a.mode == 2)
-                    {
-                      // diagonal: int phi_i^2 / dt + grad phi_i . D grad phi_i
-#pragma unroll
-                      for (int l = 0; l < N; ++l)
-#pragma unroll
-                        for (int j = 0; j < N; ++j)
-#pragma unroll
-                          for (int i = 0; i < N; ++i)
-                            {
-                              const T bx = a.B[qx * N + i], by = a.B[qy * N + j], bz = a.B[qz * N + l];
-                              const T p[3] = {a.G[qx * N + i] * a.ih[0] * by * bz, bx * a.G[qy * N + j] * a.ih[1] * bz,
-                                              bx * by * a.G[qz * N + l] * a.ih[2]};
-                              const T phi = bx * by * bz;
-                              const T pn  = p[0] * nv[0] + p[1] * nv[1] + p[2] * nv[2];
-                              const T pp  = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
-                              R[(l * N + j) * N + i] += jw * (a.inv_dt * phi * phi + a.eps_t * pp + (a.eps_n - a.eps_t) * pn * pn);
-                            }
-                      continue;
-                    }
-                  // integrand: value part and gradient part (flux)
-                  const T gn = g[0] * nv[0] + g[1] * nv[1] + g[2] * nv[2];
-                  T       val, f[3];
-                  if (a.mode == 0)
-                    {
-                      val = jw * a.inv_dt * uv;
-#pragma unroll
-                      for (int d = 0; d < 3; ++d)
-                        f[d] = jw * (a.eps_t * g[d] + (a.eps_n - a.eps_t) * gn * nv[d]);
-                    }
-                  else
-                    {
-                      val            = T(0);
-                      const T cflux = T(0.5) * (T(1) - uv * uv);
-#pragma unroll
-                      for (int d = 0; d < 3; ++d)
-                        f[d] = jw * (cflux * nv[d] - a.eps_t * g[d] - (a.eps_n - a.eps_t) * gn * nv[d]);
-                    }
+                  // int phi_i^2 / dt + grad phi_i . D grad phi_i
 #pragma unroll
                   for (int l = 0; l < N; ++l)
 #pragma unroll
@@ -162,20 +119,18 @@ namespace mpdg
                       for (int i = 0; i < N; ++i)
                         {
                           const T bx = a.B[qx * N + i], by = a.B[qy * N + j], bz = a.B[qz * N + l];
-                          R[(l * N + j) * N + i] += val * bx * by * bz + f[0] * a.G[qx * N + i] * a.ih[0] * by * bz +
-                                                    f[1] * bx * a.G[qy * N + j] * a.ih[1] * bz +
-                                                    f[2] * bx * by * a.G[qz * N + l] * a.ih[2];
+                          const T p[3] = {a.G[qx * N + i] * a.ih[0] * by * bz, bx * a.G[qy * N + j] * a.ih[1] * bz,
+                                          bx * by * a.G[qz * N + l] * a.ih[2]};
+                          const T phi = bx * by * bz;
+                          const T pn  = p[0] * nv[0] + p[1] * nv[1] + p[2] * nv[2];
+                          const T pp  = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
+                          R[(l * N + j) * N + i] += jw * (a.inv_dt * phi * phi + a.eps_t * pp + (a.eps_n - a.eps_t) * pn * pn);
                         }
                 }
 #pragma unroll
           for (int q = 0; q < N3; ++q)
             if (!con[q])
-              {
-                if (a.mode == 2)
-                  atomicAdd(a.diag + idx[q], (double)R[q]);
-                else
-                  atomicAdd(a.dst + idx[q], a.scale * R[q]);
-              }
+              atomicAdd(a.diag + idx[q], (double)R[q]);
         }
     }
 
@@ -321,6 +276,364 @@ namespace mpdg
         }
     }
 
+    // Parameters of the marching kernels
+    template <typename T, int N>
+    struct PointArgs
+    {
+      GridDesc       g;
+      SyncDesc       s;
+      GaussTab<T, N> t;
+      T              eps_t, eps;   // scale eps_t, scale (eps_n - eps_t) (scale = -1 in the right-hand side)
+      T              mass;         // scale / dt (0 in the right-hand side)
+      T              tol2, inv_tol; // normalisation: 1 / |n| where |n|^2 > tol2, else inv_tol
+      const T       *src, *b;
+      T             *dst;
+      const double  *n[3];
+      const double  *band_ls;
+      T              band;
+      int            mask_src;
+    };
+
+    // cell of a lane (a lane outside the mesh reads the fields of the nearest cell), and the values of a
+    // plainly read field at the cell's nodes or Gauss points
+    struct PointCell
+    {
+      int c[3];
+    };
+    template <typename T, int N>
+    __device__ __forceinline__ PointCell
+    point_cell(const GridDesc &g, int cx, int cy, int cz)
+    {
+      return PointCell{{min(cx, g.m[0] - 1), min(cy, g.m[1] - 1), cz}};
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    field_nodes(const double *f, const GridDesc &g, const PointCell &c, T *v)
+    {
+      constexpr int K  = N - 1;
+      const int     sy = g.n[0], sz = g.n[0] * g.n[1];
+      f += K * c.c[0] + (long long)sy * (K * c.c[1]) + (long long)sz * (K * c.c[2]);
+#pragma unroll
+      for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            v[(l * N + j) * N + i] = (T)__ldg(f + (j * sy + l * sz + i));
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    interpolate(T *v, const T *B)
+    {
+      gp_interpolate<T, N, 0>(v, B);
+      gp_interpolate<T, N, 1>(v, B);
+      gp_interpolate<T, N, 2>(v, B);
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    test(T *S, const GaussTab<T, N> &t, T *out)
+    {
+      gp_test<T, N, 2>(S, t.Bt[2]);
+      gp_test<T, N, 1>(S, t.Bt[1]);
+      gp_test<T, N, 0>(S, t.Bt[0]);
+#pragma unroll
+      for (int q = 0; q < N * N * N; ++q)
+        out[q] = S[q];
+    }
+    __device__ __forceinline__ double
+    point_rsqrt(double x)
+    {
+      return rsqrt(x);
+    }
+    __device__ __forceinline__ float
+    point_rsqrt(float x)
+    {
+      return 1.0f / sqrtf(x);
+    }
+    // points of the narrow band, one bit per Gauss point
+    template <typename T, int N, class Args>
+    __device__ __forceinline__ unsigned long long
+    band_bits(const Args &a, const PointCell &c)
+    {
+      T v[N * N * N];
+      field_nodes<T, N>(a.band_ls, a.g, c, v);
+      interpolate<T, N>(v, a.t.B);
+      unsigned long long bits = 0;
+#pragma unroll
+      for (int q = 0; q < N * N * N; ++q)
+        bits |= (unsigned long long)(fabs(v[q]) < a.band ? 1u : 0u) << q;
+      return bits;
+    }
+
+    // reinitialisation tangent (RHS = false) and right-hand side (RHS = true: src = psi_old, the flux
+    // (1 - psi^2) / 2 n - D grad psi, eps_t and eps with a minus sign), one plane of Gauss points at a time
+    template <int K, typename T, bool RHS>
+    struct ReinitCellOp
+    {
+      static constexpr int  N = K + 1, N2 = N * N, N3 = N * N * N;
+      static constexpr bool HEAVY = true, NODES = true;
+      const PointArgs<T, N> &a;
+      __device__ __forceinline__ PointCell
+      load(bool, int cx, int cy, int cz) const
+      {
+        return point_cell<T, N>(a.g, cx, cy, cz);
+      }
+      __device__ __forceinline__ void
+      apply(T *R, const MarchNodes<K, T> &nodes, const PointCell &c) const
+      {
+        const int       sy = a.g.n[0], sz = a.g.n[0] * a.g.n[1];
+        const long long first = K * c.c[0] + (long long)sy * (K * c.c[1]) + (long long)sz * (K * c.c[2]);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          R[q] = T(0);
+#pragma unroll(K == 1 ? 2 : 1)
+        for (int qz = 0; qz < N; ++qz)
+          {
+            const T *bz = a.t.B + qz * N, *gz = a.t.Gz + qz * (N - 1);
+            T        v[3][N2], u[N2], F[N2], S[N2], G[N2];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+              {
+                const double *f = a.n[d] + first;
+                pl_nodes<T, N>([&](int l, int j, int i) { return (T)__ldg(f + (j * sy + l * sz + i)); }, bz, gz, v[d], (T *)nullptr);
+                pl_interpolate<T, N>(v[d], a.t.B);
+              }
+            pl_nodes<T, N>([&](int l, int j, int i) { return nodes.row[l * N + j][i]; }, bz, gz, u, F);
+            pl_interpolate<T, N>(u, a.t.B);
+            pl_interpolate<T, N>(F, a.t.B);
+            // the flux's factor of n_h: c = eps (n_h . grad u) / |n_h|^2, in the right-hand side with the
+            // compressive part (1 - psi^2) / (2 |n_h|)
+#pragma unroll
+            for (int p = 0; p < N2; ++p)
+              {
+                const T gx = gp_derivative<T, N, 0>(u, a.t.D[0], p), gy = gp_derivative<T, N, 1>(u, a.t.D[1], p);
+                const T nn = fma(v[2][p], v[2][p], fma(v[1][p], v[1][p], v[0][p] * v[0][p]));
+                const T inv = nn > a.tol2 ? point_rsqrt(nn) : a.inv_tol;
+                const T an  = a.eps * (fma(v[2][p], F[p], fma(v[1][p], gy, v[0][p] * gx)) * inv);
+                G[p]        = RHS ? inv * (T(0.5) * (T(1) - u[p] * u[p]) + an) : inv * an;
+                S[p]        = a.mass * u[p];
+                F[p]        = fma(a.eps_t, F[p], G[p] * v[2][p]);
+              }
+            pl_divergence<T, N, 0>(S, a.t.P[0], [&](int p) { return fma(a.eps_t, gp_derivative<T, N, 0>(u, a.t.D[0], p), G[p] * v[0][p]); });
+            pl_divergence<T, N, 1>(S, a.t.P[1], [&](int p) { return fma(a.eps_t, gp_derivative<T, N, 1>(u, a.t.D[1], p), G[p] * v[1][p]); });
+            pl_test<T, N>(S, F, a.t, qz, R);
+          }
+      }
+    };
+
+    // M / dt + eps K in a narrow band (isotropic, no normal field): value and flux masked per Gauss point
+    template <int K, typename T>
+    struct BandCellOp
+    {
+      static constexpr bool HEAVY = false, NODES = false;
+      static constexpr int N = K + 1, N3 = N * N * N;
+      const PointArgs<T, N> &a;
+      __device__ __forceinline__ PointCell
+      load(bool, int cx, int cy, int cz) const
+      {
+        return point_cell<T, N>(a.g, cx, cy, cz);
+      }
+      template <bool DOT>
+      __device__ __forceinline__ double
+      apply(T *u, const PointCell &c) const
+      {
+        T                        S[N3];
+        const unsigned long long bits = band_bits<T, N>(a, c);
+        auto in = [&](int q, T x) { return (bits >> q) & 1u ? x : T(0); };
+        interpolate<T, N>(u, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          S[q] = in(q, a.mass * u[q]);
+        // t.D carries the diffusivity
+        gp_divergence<T, N, 0>(S, a.t.P[0], [&](int q) { return in(q, gp_derivative<T, N, 0>(u, a.t.D[0], q)); });
+        gp_divergence<T, N, 1>(S, a.t.P[1], [&](int q) { return in(q, gp_derivative<T, N, 1>(u, a.t.D[1], q)); });
+        gp_divergence<T, N, 2>(S, a.t.P[2], [&](int q) { return in(q, gp_derivative<T, N, 2>(u, a.t.D[2], q)); });
+        test<T, N>(S, a.t, u);
+        return 0.0;
+      }
+    };
+
+    // int (grad psi)_DIR phi, in the band if there is one; NORMALIZED: the unit gradient (|.| > 1e-16)
+    template <int K, int DIR, bool NORMALIZED>
+    struct GradientCellOp
+    {
+      static constexpr bool HEAVY = false, NODES = false;
+      static constexpr int N = K + 1, N3 = N * N * N;
+      const PointArgs<double, N> &a;
+      __device__ __forceinline__ PointCell
+      load(bool, int cx, int cy, int cz) const
+      {
+        return point_cell<double, N>(a.g, cx, cy, cz);
+      }
+      template <bool DOT>
+      __device__ __forceinline__ double
+      apply(double *u, const PointCell &c) const
+      {
+        double             S[N3];
+        unsigned long long bits = ~0ull;
+        if (a.band_ls)
+          bits = band_bits<double, N>(a, c);
+        interpolate<double, N>(u, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          {
+            double g = gp_derivative<double, N, DIR>(u, a.t.D[DIR], q);
+            if constexpr (NORMALIZED)
+              {
+                constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
+                const double  g1 = gp_derivative<double, N, D1>(u, a.t.D[D1], q), g2 = gp_derivative<double, N, D2>(u, a.t.D[D2], q);
+                const double  nn = sqrt(g * g + g1 * g1 + g2 * g2);
+                g *= nn > 1e-16 ? 1.0 / nn : 1e16;
+              }
+            S[q] = (bits >> q) & 1u ? g : 0.0;
+          }
+        test<double, N>(S, a.t, u);
+        return 0.0;
+      }
+    };
+
+    // -int div(n) phi, n = normalize(n_i, tol) at every DoF; the marching input is n_x.  t.D carries the sign.
+    template <int K>
+    struct DivergenceCellOp
+    {
+      static constexpr bool HEAVY = false, NODES = false;
+      static constexpr int N = K + 1, N3 = N * N * N;
+      const PointArgs<double, N> &a;
+      __device__ __forceinline__ PointCell
+      load(bool, int cx, int cy, int cz) const
+      {
+        return point_cell<double, N>(a.g, cx, cy, cz);
+      }
+      template <bool DOT>
+      __device__ __forceinline__ double
+      apply(double *u, const PointCell &c) const
+      {
+        double S[N3], inv[N3], v[N3];
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          inv[q] = u[q] * u[q];
+        field_nodes<double, N>(a.n[1], a.g, c, v);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          inv[q] = fma(v[q], v[q], inv[q]);
+        field_nodes<double, N>(a.n[2], a.g, c, v);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          {
+            const double nn = fma(v[q], v[q], inv[q]);
+            inv[q]          = nn > a.tol2 ? point_rsqrt(nn) : a.inv_tol;
+            v[q] *= inv[q];
+            u[q] *= inv[q];
+          }
+        interpolate<double, N>(v, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          S[q] = gp_derivative<double, N, 2>(v, a.t.D[2], q);
+        interpolate<double, N>(u, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          S[q] += gp_derivative<double, N, 0>(u, a.t.D[0], q);
+        field_nodes<double, N>(a.n[1], a.g, c, v);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          v[q] *= inv[q];
+        interpolate<double, N>(v, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          S[q] += gp_derivative<double, N, 1>(v, a.t.D[1], q);
+        if (a.band_ls)
+          {
+            const unsigned long long bits = band_bits<double, N>(a, c);
+#pragma unroll
+            for (int q = 0; q < N3; ++q)
+              S[q] = (bits >> q) & 1u ? S[q] : 0.0;
+          }
+        test<double, N>(S, a.t, u);
+        return 0.0;
+      }
+    };
+
+#ifndef MPDG_REINIT_MINB
+#define MPDG_REINIT_MINB 0
+#endif
+    // CTAs (of 128 threads) per SM the register allocation is held to
+    template <int K, typename T, bool HEAVY>
+    struct PointMinBlocks
+    {
+      static constexpr int value = MPDG_REINIT_MINB ? MPDG_REINIT_MINB : K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? (HEAVY ? 2 : 3) : 4) : 2);
+    };
+
+    template <int K, typename T, OutMode MODE, class Op>
+    __global__ void __launch_bounds__(MARCH_NT, PointMinBlocks<K, T, Op::HEAVY>::value)
+    reinit_march_kernel(const __grid_constant__ PointArgs<T, K + 1> a)
+    {
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      __shared__ unsigned                        s_ticket;
+      __shared__ __align__(8) unsigned long long s_bars[2];
+      Op                                         op{a};
+      march_body<K, T, MODE, Op, false, true>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
+                                              reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
+    }
+
+    template <int K, typename T, OutMode MODE, class Op>
+    cudaError_t
+    launch_point_kernel(PointArgs<T, K + 1> &a, cudaStream_t s)
+    {
+      auto                                   kern = reinit_march_kernel<K, T, MODE, Op>;
+      static std::atomic<unsigned long long> devices{0};
+      constexpr size_t                       bytes = MarchLayout<K, T>::bytes;
+      if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
+        return e;
+      const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, PointMinBlocks<K, T, Op::HEAVY>::value);
+      kern<<<ctas, MARCH_NT, bytes, s>>>(a);
+      return cudaGetLastError();
+    }
+
+    // the tangent (mode 0), the banded isotropic form (mode 0 without a normal field) or the rhs (mode 1)
+    template <int K, typename T>
+    cudaError_t
+    launch_reinit_march(const ReinitLaunch<T> &h, int mode, cudaStream_t s)
+    {
+      constexpr int       N = K + 1;
+      PointArgs<T, N>     a{};
+      const Tables1D     &t = tables(K);
+      const bool          banded = h.band > 0.0 && h.band_ls != nullptr;
+      a.g                        = h.grid;
+      a.s                        = h.sync;
+      a.t.fill(t, h.hlen);
+      if (h.normal[0] == nullptr) // the banded form's flux: D carries the diffusivity
+        for (int d = 0; d < 3; ++d)
+          gp_on_differences<T, N>(t.Dq, h.scale * h.eps_tangential / h.hlen[d], a.t.D[d]);
+      a.eps_t    = (T)((mode == 1 ? -1.0 : h.scale) * h.eps_tangential);
+      a.eps      = (T)((mode == 1 ? -1.0 : h.scale) * (h.eps_normal - h.eps_tangential));
+      a.mass     = mode == 1 ? T(0) : (T)(h.scale / h.dt);
+      a.tol2     = (T)(h.normal_tolerance * h.normal_tolerance);
+      a.inv_tol  = (T)(1.0 / h.normal_tolerance);
+      a.src      = h.src;
+      a.dst      = h.dst;
+      a.b        = h.b;
+      a.mask_src = mode == 1 ? 0 : h.mask_src;
+      a.band_ls  = banded ? h.band_ls : nullptr;
+      a.band     = (T)h.band;
+      for (int d = 0; d < 3; ++d)
+        a.n[d] = h.normal[d];
+      if (mode == 1)
+        return launch_point_kernel<K, T, OutMode::Set, ReinitCellOp<K, T, true>>(a, s);
+      if (h.normal[0] == nullptr)
+        switch (h.out_mode)
+          {
+            case 0: return launch_point_kernel<K, T, OutMode::Set, BandCellOp<K, T>>(a, s);
+            case 1: return launch_point_kernel<K, T, OutMode::Add, BandCellOp<K, T>>(a, s);
+            default: return launch_point_kernel<K, T, OutMode::BPlus, BandCellOp<K, T>>(a, s);
+          }
+      switch (h.out_mode)
+        {
+          case 0: return launch_point_kernel<K, T, OutMode::Set, ReinitCellOp<K, T, false>>(a, s);
+          case 1: return launch_point_kernel<K, T, OutMode::Add, ReinitCellOp<K, T, false>>(a, s);
+          default: return launch_point_kernel<K, T, OutMode::BPlus, ReinitCellOp<K, T, false>>(a, s);
+        }
+    }
+
     template <int K, typename T>
     cudaError_t
     launch_reinit(const ReinitLaunch<T> &h, int mode, cudaStream_t s)
@@ -390,8 +703,10 @@ namespace mpdg
         }
       const long long ncell  = (long long)h.grid.m[0] * h.grid.m[1] * h.grid.m[2];
       const int       blocks = (int)std::max<long long>(1, std::min<long long>((ncell + 127) / 128, 148LL * 16));
-      if (!h.faces_only)
-        reinit_kernel<K, T><<<blocks, 128, 0, s>>>(a);
+      if (mode == 2)
+        reinit_diag_kernel<K, T><<<blocks, 128, 0, s>>>(a);
+      else if (cudaError_t e = launch_reinit_march<K, T>(h, mode, s); e != cudaSuccess)
+        return e;
       if (h.wetting && a.n[0] != nullptr)
         {
           cudaError_t e = cudaGetLastError();
@@ -405,190 +720,72 @@ namespace mpdg
 
   namespace
   {
-    // Right-hand sides of the normal-vector and curvature projections (one thread per cell):
-    //   mode 0: dst_d += int g_d phi, g = grad psi, or normalize(grad psi, 1e-16) when normalized
-    //           (normal_vector_operator.cpp:160-240, no narrow band)
-    //   mode 1: dst   += -int div(n) phi with n = normalize(n_i, tol) at every DoF
-    //           (curvature_operator.cpp:190-255, no narrow band)
-    template <int K>
-    __global__ void __launch_bounds__(128)
-    level_set_rhs_kernel(const GridDesc g, const double *B, const double *G, const double *w, double det, double ihx,
-                         double ihy, double ihz, int mode, int normalized, double tol, const double *in0,
-                         const double *in1, const double *in2, double *out0, double *out1, double *out2,
-                         const double *band_ls, double band)
+    template <int K, bool NORMALIZED>
+    cudaError_t
+    launch_normal_rhs(PointArgs<double, K + 1> &a, double *const out[3], cudaStream_t s)
     {
-      constexpr int   N = K + 1, N3 = N * N * N;
-      const double    ih[3] = {ihx, ihy, ihz};
-      const int       m0 = g.m[0], m1 = g.m[1];
-      const long long ncell = (long long)m0 * m1 * g.m[2];
-      for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncell; c += (long long)gridDim.x * blockDim.x)
-        {
-          const int cx = (int)(c % m0), cy = (int)((c / m0) % m1), cz = (int)(c / ((long long)m0 * m1));
-          long long idx[N3];
-          bool      con[N3];
-          double    v[3][N3], R[3][N3], ls[N3];
-#pragma unroll
-          for (int l = 0; l < N; ++l)
-#pragma unroll
-            for (int j = 0; j < N; ++j)
-#pragma unroll
-              for (int i = 0; i < N; ++i)
-                {
-                  const int       q = (l * N + j) * N + i;
-                  const int       I = K * cx + i, J = K * cy + j, L = K * cz + l;
-                  const long long id = (long long)I + (long long)g.n[0] * ((long long)J + (long long)g.n[1] * L);
-                  idx[q]            = id;
-                  con[q]            = is_constrained(g, I, J, L, id);
-                  ls[q]             = band_ls ? band_ls[id] : 0.0;
-                  if (mode == 0)
-                    v[0][q] = in0[id];
-                  else
-                    {
-                      const double a = in0[id], b = in1[id], e = in2[id];
-                      const double nn = sqrt(a * a + b * b + e * e), s = nn > tol ? 1.0 / nn : 1.0 / tol;
-                      v[0][q] = a * s, v[1][q] = b * s, v[2][q] = e * s;
-                    }
-#pragma unroll
-                  for (int d = 0; d < 3; ++d)
-                    R[d][q] = 0.0;
-                }
-          for (int qz = 0; qz < N; ++qz)
-            for (int qy = 0; qy < N; ++qy)
-              for (int qx = 0; qx < N; ++qx)
-                {
-                  double gv[3] = {0.0, 0.0, 0.0}, div = 0.0, lq = 0.0;
-#pragma unroll
-                  for (int l = 0; l < N; ++l)
-#pragma unroll
-                    for (int j = 0; j < N; ++j)
-#pragma unroll
-                      for (int i = 0; i < N; ++i)
-                        {
-                          const int    q  = (l * N + j) * N + i;
-                          const double bx = B[qx * N + i], by = B[qy * N + j], bz = B[qz * N + l];
-                          const double p[3] = {G[qx * N + i] * ih[0] * by * bz, bx * G[qy * N + j] * ih[1] * bz,
-                                               bx * by * G[qz * N + l] * ih[2]};
-                          lq += bx * by * bz * ls[q];
-                          if (mode == 0)
-                            {
-#pragma unroll
-                              for (int d = 0; d < 3; ++d)
-                                gv[d] += p[d] * v[0][q];
-                            }
-                          else
-                            div += p[0] * v[0][q] + p[1] * v[1][q] + p[2] * v[2][q];
-                        }
-                  // narrow band (normal_vector_operator.cpp:184-191, curvature_operator.cpp:209-214):
-                  // the gradient (before its normalisation) or the divergence is masked by
-                  // |level set| < band at the point
-                  if (band_ls && !(fabs(lq) < band))
-                    {
-                      gv[0] = gv[1] = gv[2] = 0.0;
-                      div                   = 0.0;
-                    }
-                  if (mode == 0 && normalized)
-                    {
-                      const double nn = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
-                      const double s  = nn > 1e-16 ? 1.0 / nn : 1e16;
-#pragma unroll
-                      for (int d = 0; d < 3; ++d)
-                        gv[d] *= s;
-                    }
-                  const double jw = det * w[qx] * w[qy] * w[qz];
-#pragma unroll
-                  for (int l = 0; l < N; ++l)
-#pragma unroll
-                    for (int j = 0; j < N; ++j)
-#pragma unroll
-                      for (int i = 0; i < N; ++i)
-                        {
-                          const double phi = B[qx * N + i] * B[qy * N + j] * B[qz * N + l] * jw;
-                          if (mode == 0)
-                            {
-#pragma unroll
-                              for (int d = 0; d < 3; ++d)
-                                R[d][(l * N + j) * N + i] += gv[d] * phi;
-                            }
-                          else
-                            R[0][(l * N + j) * N + i] -= div * phi;
-                        }
-                }
-#pragma unroll
-          for (int q = 0; q < N3; ++q)
-            if (!con[q])
-              {
-                atomicAdd(out0 + idx[q], R[0][q]);
-                if (mode == 0)
-                  {
-                    atomicAdd(out1 + idx[q], R[1][q]);
-                    atomicAdd(out2 + idx[q], R[2][q]);
-                  }
-              }
-        }
+      cudaError_t e;
+      a.dst = out[0];
+      if ((e = launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 0, NORMALIZED>>(a, s)) != cudaSuccess)
+        return e;
+      a.dst = out[1];
+      if ((e = launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 1, NORMALIZED>>(a, s)) != cudaSuccess)
+        return e;
+      a.dst = out[2];
+      return launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 2, NORMALIZED>>(a, s);
     }
 
-    // 1-D tables of degree K in device memory for the level-set rhs kernels (uploaded once per device)
-    const double *
-    level_set_tables(int K)
+    template <int K>
+    cudaError_t
+    launch_level_set_rhs(const GridDesc &g, const SyncDesc &sync, const double hlen[3], int mode, int normalized, double tol,
+                         const double *const in[3], double *const out[3], cudaStream_t s, const double *band_ls,
+                         double band)
     {
-      static std::mutex mtx;
-      static double    *dev[64][3] = {}; // [device][degree]
-      int               d          = 0;
-      if (cudaGetDevice(&d) != cudaSuccess || d >= 64)
-        return nullptr;
-      std::lock_guard<std::mutex> lock(mtx);
-      if (!dev[d][K])
+      constexpr int        N = K + 1;
+      PointArgs<double, N> a{};
+      a.g = g;
+      a.s = sync;
+      a.t.fill(tables(K), hlen);
+      a.src      = in[0];
+      a.mask_src = 0;
+      a.band_ls  = band > 0.0 ? band_ls : nullptr;
+      a.band     = band;
+      if (mode == 0)
+        return normalized ? launch_normal_rhs<K, true>(a, out, s) : launch_normal_rhs<K, false>(a, out, s);
+      for (int d = 0; d < 3; ++d)
         {
-          const Tables1D &t = tables(K);
-          const int       n = t.n;
-          double          h[3 * MAX_N * MAX_N]{};
-          for (int i = 0; i < n * n; ++i)
-            {
-              h[i]         = t.B[i];
-              h[n * n + i] = t.G[i];
-            }
-          for (int q = 0; q < n; ++q)
-            h[2 * n * n + q] = t.qw[q];
-          double *p = nullptr;
-          // a legacy-stream copy, completed before kernels on other streams read the table
-          if (cudaMalloc(&p, sizeof(h)) != cudaSuccess || cudaMemcpy(p, h, sizeof(h), cudaMemcpyHostToDevice) != cudaSuccess ||
-              cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
-            return nullptr;
-          dev[d][K] = p;
+          a.n[d] = in[d];
+          for (int i = 0; i < N * (N - 1); ++i)
+            a.t.D[d][i] = -a.t.D[d][i];
         }
-      return dev[d][K];
+      a.tol2    = tol * tol;
+      a.inv_tol = 1.0 / tol;
+      a.dst     = out[0];
+      return launch_point_kernel<K, double, OutMode::Set, DivergenceCellOp<K>>(a, s);
     }
   } // namespace
 
+  // Right-hand sides of the normal-vector and curvature projections:
+  //   mode 0: dst_d += int g_d phi, g = grad psi, or normalize(grad psi, 1e-16) when normalized
+  //           (normal_vector_operator.cpp:160-240), one launch per component
+  //   mode 1: dst   = -int div(n) phi with n = normalize(n_i, tol) at every DoF
+  //           (curvature_operator.cpp:190-255)
+  // Narrow band (normal_vector_operator.cpp:184-191, curvature_operator.cpp:209-214): the gradient or the
+  // divergence is masked by |level set| < band at the Gauss point.
   cudaError_t
-  level_set_rhs(const GridDesc &g, int K, const double hlen[3], int mode, int normalized, double tol,
+  level_set_rhs(const GridDesc &g, const SyncDesc &sync, int K, const double hlen[3], int mode, int normalized, double tol,
                 const double *in0, const double *in1, const double *in2, double *out0, double *out1, double *out2,
                 cudaStream_t s, const double *band_ls, double band)
   {
-    if (!(band > 0.0))
-      band_ls = nullptr;
-    if (K < 1 || K > 3)
-      return cudaErrorInvalidValue;
-    const double *tab = level_set_tables(K);
-    if (!tab)
-      return cudaErrorMemoryAllocation;
-    const int       n      = K + 1;
-    const long long ncell  = (long long)g.m[0] * g.m[1] * g.m[2];
-    const int       blocks = (int)std::max<long long>(1, std::min<long long>((ncell + 127) / 128, 148LL * 16));
-    const double    det    = hlen[0] * hlen[1] * hlen[2];
-    if (K == 1)
-      level_set_rhs_kernel<1><<<blocks, 128, 0, s>>>(g, tab, tab + n * n, tab + 2 * n * n, det, 1.0 / hlen[0],
-                                                      1.0 / hlen[1], 1.0 / hlen[2], mode, normalized, tol, in0, in1,
-                                                      in2, out0, out1, out2, band_ls, band);
-    else if (K == 2)
-      level_set_rhs_kernel<2><<<blocks, 128, 0, s>>>(g, tab, tab + n * n, tab + 2 * n * n, det, 1.0 / hlen[0],
-                                                      1.0 / hlen[1], 1.0 / hlen[2], mode, normalized, tol, in0, in1,
-                                                      in2, out0, out1, out2, band_ls, band);
-    else
-      level_set_rhs_kernel<3><<<blocks, 128, 0, s>>>(g, tab, tab + n * n, tab + 2 * n * n, det, 1.0 / hlen[0],
-                                                      1.0 / hlen[1], 1.0 / hlen[2], mode, normalized, tol, in0, in1,
-                                                      in2, out0, out1, out2, band_ls, band);
-    return cudaGetLastError();
+    const double *in[3]  = {in0, in1, in2};
+    double       *out[3] = {out0, out1, out2};
+    switch (K)
+      {
+        case 1: return launch_level_set_rhs<1>(g, sync, hlen, mode, normalized, tol, in, out, s, band_ls, band);
+        case 2: return launch_level_set_rhs<2>(g, sync, hlen, mode, normalized, tol, in, out, s, band_ls, band);
+        case 3: return launch_level_set_rhs<3>(g, sync, hlen, mode, normalized, tol, in, out, s, band_ls, band);
+        default: return cudaErrorInvalidValue;
+      }
   }
 
   template <typename T>
