@@ -90,7 +90,6 @@ struct mpdg_op
   bool          solid = false;    // temperature-dependent material (heat, FE_Q(1, 2))
   SolidMaterial smat{};
   const double *d_temp_old = nullptr; // T_old of the solidification tangent (not owned)
-  long long     sync_cap = 0;         // brick flags allocated in d_sync (after the 3 counters)
   int           supg = 0;         // SUPG stabilisation (advection-diffusion)
   // inflow/outflow condition (advection-diffusion): inflow DoFs are identity rows of vmult
   uint8_t      *d_mask_io  = nullptr; // Dirichlet mask | inflow flags: the apply's read / write mask
@@ -312,8 +311,7 @@ namespace
   }
 
   // Temperature-dependent material: the tangent (rhs = false) or the residual part of create_rhs
-  // (rhs = true, dst +=, src unused) with the operator's temperature and old temperature.  FP32
-  // applies read FP32 copies of both.
+  // (rhs = true, dst +=, src unused) with the operator's temperature and old temperature.
   template <typename T>
   int
   solid_apply(mpdg_op *op, int mode, double scale, T *dst, const T *src, const T *b, int mask_src, const int *skip,
@@ -333,26 +331,9 @@ namespace
       h.hlen[d] = op->h[d];
     h.mat  = op->smat;
     h.grid = op->grid<T>();
-    int shape[3];
-    heat_solid_brick_shape<T>(op->degree, shape);
-    for (int d = 0; d < 3; ++d)
-      h.grid.nbr[d] = (op->m[d] + shape[d] - 1) / shape[d];
-    h.sync = op->sync();
-    if constexpr (std::is_same<T, double>::value)
-      {
-        h.temp     = t64;
-        h.temp_old = to64;
-      }
-    else
-      {
-        T *t32 = op->vec<T>("solid_t32"), *to32 = op->vec<T>("solid_to32");
-        if (!t32 || !to32)
-          return fail(MPDG_ERR_NOMEM, "FP32 temperature copies");
-        MPDG_CUDA(vec_convert<T, double>(t32, t64, op->ndofs, op->stream));
-        MPDG_CUDA(vec_convert<T, double>(to32, to64, op->ndofs, op->stream));
-        h.temp     = t32;
-        h.temp_old = to32;
-      }
+    h.sync     = op->sync();
+    h.temp     = t64;
+    h.temp_old = to64;
     h.src      = src;
     h.dst      = dst;
     h.b        = b;
@@ -536,8 +517,7 @@ namespace
           return fail(MPDG_ERR_NOMEM, "diagonal work vector");
         if (op->solid)
           {
-            MPDG_CUDA(vec_fill<double>(d64, 0.0, op->ndofs, op->stream));
-            MPDG_CUDA(heat_solid_diagonal(g, op->degree, op->smat, op->dt, op->h, op->d_temp, op->d_temp_old, d64,
+            MPDG_CUDA(heat_solid_diagonal(g, op->sync(), op->degree, op->smat, op->dt, op->h, op->d_temp, op->d_temp_old, d64,
                                           op->stream));
             MPDG_CUDA(vec_set_constrained<double>(d64, 1.0, g, op->stream));
           }
@@ -1152,7 +1132,6 @@ mpdg_op_create(const mpdg_mesh_desc *mesh, const mpdg_op_params *params, mpdg_op
     return clean(MPDG_ERR_NOMEM, "device allocation in mpdg_op_create");
   if (op->kind == MPDG_HEAT && cudaMalloc(&op->d_part, sizeof(double) * nbrk) != cudaSuccess)
     return clean(MPDG_ERR_NOMEM, "fused dot partials");
-  op->sync_cap = nbrk;
   if (cudaMemset(op->d_sync, 0, sizeof(unsigned) * (3 + nbrk)) != cudaSuccess ||
       cudaMemset(op->d_err, 0, sizeof(int)) != cudaSuccess)
     return clean(MPDG_ERR_CUDA, "cudaMemset in mpdg_op_create");
@@ -1331,24 +1310,6 @@ mpdg_op_set_solidification(mpdg_op *op, const mpdg_solid_liquid *mat)
       (!mat->sharp && !(mat->liquidus_temperature > mat->solidus_temperature)) || !(mat->latent_heat >= 0.0) ||
       mat->capacity_type < 0 || mat->capacity_type > 2)
     return fail(MPDG_ERR_ARG, "material parameters must be positive and the liquidus above the solidus");
-  // the solid-phase kernel's bricks may outnumber the flags allocated for the constant-material ones
-  int shape[3];
-  heat_solid_brick_shape<float>(op->degree, shape);
-  long long nb = 1;
-  for (int d = 0; d < 3; ++d)
-    nb *= (op->m[d] + shape[d] - 1) / shape[d];
-  if (nb > op->sync_cap)
-    {
-      unsigned *fresh = nullptr;
-      MPDG_CUDA(cudaStreamSynchronize(op->stream));
-      if (cudaMalloc(&fresh, sizeof(unsigned) * (3 + nb)) != cudaSuccess)
-        return fail(MPDG_ERR_NOMEM, "brick flags");
-      MPDG_CUDA(cudaMemsetAsync(fresh, 0, sizeof(unsigned) * (3 + nb), op->stream));
-      MPDG_CUDA(cudaFree(op->d_sync));
-      op->d_sync   = fresh;
-      op->sync_cap = nb;
-      op->epoch    = 0;
-    }
   SolidMaterial m;
   m.rho_l      = mat->liquid_density;
   m.cp_l       = mat->liquid_specific_heat;

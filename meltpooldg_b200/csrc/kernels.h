@@ -98,11 +98,11 @@ namespace mpdg
     double        dt     = 1.0;
     double        hlen[3]{};
     SolidMaterial mat{};
-    GridDesc      grid{};         // nbr from heat_solid_brick_shape
-    SyncDesc      sync{};
+    GridDesc      grid{};
+    SyncDesc      sync{};         // flags: adv_flags
     const T      *src      = nullptr;
-    const T      *temp     = nullptr; // linearisation temperature (plain reads)
-    const T      *temp_old = nullptr;
+    const double *temp     = nullptr; // linearisation temperature (plain reads)
+    const double *temp_old = nullptr;
     T            *dst      = nullptr;
     const T      *b        = nullptr;
     int           mask_src = 1;
@@ -110,12 +110,11 @@ namespace mpdg
   };
 
   template <typename T>
-  void heat_solid_brick_shape(int K, int shape[3]);
-  template <typename T>
   cudaError_t heat_solid_apply(const HeatSolidLaunch<T> &h, cudaStream_t s);
-  // adds the tangent's diagonal on the free rows of diag (FP64)
-  cudaError_t heat_solid_diagonal(const GridDesc &g, int K, const SolidMaterial &mat, double dt, const double hlen[3],
-                                  const double *temp, const double *temp_old, double *diag, cudaStream_t s);
+  // diag = the tangent's diagonal (FP64), constrained rows 0
+  cudaError_t heat_solid_diagonal(const GridDesc &g, const SyncDesc &sync, int K, const SolidMaterial &mat, double dt,
+                                  const double hlen[3], const double *temp, const double *temp_old, double *diag,
+                                  cudaStream_t s);
 
   // ---- conservative level-set reinitialisation (Olsson, reinit.cu), FE_Q(1, 2)
   template <typename T>
