@@ -895,18 +895,33 @@ namespace mpdg
     tiles_y      = (m[1] + TY - 1) / TY;
     // CTAs resident per SM from the shared memory footprint (227 KB usable per CTA, 228 KB per SM)
     const int per_sm = std::max(1, (int)(233472 / (smem_bytes() + 1024)));
-    // one CTA per resident slot, each with an equal share of the columns' layers; a share below
-    // four layers would spend more on its halo layer than it saves, so small lattices use fewer CTAs
-    // (at 48^3 a floor of 8 or 16 layers measured 1.5x / 2.5x slower: more CTAs win down to 4)
     layers = (long long)tiles_x * tiles_y * m[2];
-    ntiles = (int)std::max(1LL, std::min((long long)sm_count * per_sm, layers / 4));
+    const long long slots = (long long)sm_count * per_sm, ncol = (long long)tiles_x * tiles_y;
+    // Small lattices: one piece per CTA, as low as the slots allow.  A piece of h layers takes h + 1 (its halo
+    // layer) and the staging ramp however many CTAs run, so the lowest piece wins although its halo layers
+    // are redundant work (32^3 in FP64, 4 layers on 32 CTAs -> 1 layer on 128: 49.9 -> 31.4 ms for 18 solves;
+    // 48^3 in FP32, 4 -> 2 layers: mixed solve 6.4 -> 4.9 ms).  Above 4 layers a piece the equal shares below
+    // are the better cut, and below it they are not: they leave CTAs with two pieces (64^3 in FP32, 512
+    // layers on 128 or 148 CTAs: 8.6 against 9.7 ms).
+    for (int h = 1; h <= 4; ++h)
+      if (ncol * ((m[2] + h - 1) / h) <= slots)
+        {
+          slab = h;
+          range.assign(1, 0);
+          for (int z0 = 0; z0 < m[2]; z0 += h)
+            for (long long c = 0; c < ncol; ++c)
+              range.push_back(range.back() + std::min(h, m[2] - z0));
+          ntiles = (int)range.size() - 1;
+          return;
+        }
+    // Otherwise one CTA per resident slot, each with an equal share of the columns' layers
+    ntiles = (int)std::max(1LL, std::min(slots, layers / 4));
     // slabs about one share high, so that the CTAs working at the same time hold neighbouring
     // columns at about the same layers and read each other's halo planes from L2
     slab = (int)std::max(1LL, std::min((long long)m[2], (layers + ntiles / 2) / ntiles));
     // ranges of equal cost: a piece costs its layers plus about 1.5 (its halo layer and the
     // staging ramp), so CTAs whose range is cut into short pieces (the last, lower slab) take
     // fewer layers; the smallest cost bound that needs at most ntiles ranges, by bisection
-    const long long ncol = (long long)tiles_x * tiles_y;
     auto greedy = [&](double bound, std::vector<long long> *out) {
       long long n = 0, pos = 0;
       double    cost = 0.0;
