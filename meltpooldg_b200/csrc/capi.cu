@@ -130,6 +130,7 @@ struct mpdg_op
   // copy streams and events of the slab-pipelined host-buffer apply (created on first use)
   cudaStream_t             s_h2d = nullptr, s_d2h = nullptr;
   std::vector<cudaEvent_t> ev;
+  cudaEvent_t              ev_gmres[2] = {}; // the two slots of GMRES' Hessenberg columns (created on first use)
 
   template <typename T = double>
   GridDesc
@@ -903,7 +904,10 @@ namespace
     Control             ctl{max_it, abs_tol, rel_tol};
     int                 it = 0, state = 0;
     double              res0 = 0.0, res = 0.0;
-    bool                first = true;
+    bool                first = true, stopped = false;
+    for (cudaEvent_t &e : op->ev_gmres)
+      if (!e)
+        MPDG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     const Reducer       red   = op->reducer();
     auto fetch = [&](int cnt) -> int {
       MPDG_CUDA(cudaMemcpyAsync(op->h_scal, d_h, sizeof(double) * cnt, cudaMemcpyDeviceToHost, op->stream));
@@ -929,56 +933,71 @@ namespace
         state = ctl.check(it, beta);
         if (state != 0)
           break;
-        MPDG_CUDA(vec_axpby<T>(V[0], 1.0 / beta, V[0], 0.0, nullptr, n, op->stream));
+        MPDG_CUDA(gmres_next<T>(V[0], z, invd, d_h, n, op->stream));
         std::fill(g.begin(), g.end(), 0.0);
         std::fill(H.begin(), H.end(), 0.0);
-        g[0]  = beta;
-        int j = 0;
-        for (; j < m; ++j)
+        g[0] = beta;
+        // Column j of the Hessenberg matrix reaches the host while the device already works on column j + 1:
+        // its launches need no host scalar (the norm that scales the next basis vector is read on the device),
+        // so the device never waits for the host's rotations.  The price is one discarded column per
+        // solve.  Two pinned slots of 32 scalars are taken in turn.
+        auto column = [&](int jc) -> int {
+          MPDG_CUDA(cudaEventSynchronize(op->ev_gmres[jc & 1]));
+          const double *hc = op->h_scal + 32 * (jc & 1);
+          ++it;
+          const double hn = std::sqrt(std::max(0.0, hc[jc + 1]));
+          for (int i = 0; i <= jc; ++i)
+            H[i * m + jc] = hc[i];
+          H[(jc + 1) * m + jc] = hn;
+          for (int i = 0; i < jc; ++i)
+            {
+              const double t0 = H[i * m + jc], t1 = H[(i + 1) * m + jc];
+              H[i * m + jc]       = cs[i] * t0 + sn[i] * t1;
+              H[(i + 1) * m + jc] = -sn[i] * t0 + cs[i] * t1;
+            }
+          const double a = H[jc * m + jc], c = H[(jc + 1) * m + jc];
+          const double r = std::hypot(a, c);
+          cs[jc]              = a / r;
+          sn[jc]              = c / r;
+          H[jc * m + jc]       = r;
+          H[(jc + 1) * m + jc] = 0.0;
+          g[jc + 1]            = -sn[jc] * g[jc];
+          g[jc]                = cs[jc] * g[jc];
+          res                  = std::abs(g[jc + 1]);
+          hist.push_back(res);
+          state   = ctl.check(it, res);
+          stopped = state != 0 || hn == 0.0;
+          return MPDG_OK;
+        };
+        int j   = 0; // columns taken
+        stopped = false;
+        for (int jn = 0; jn < m && !stopped; ++jn)
           {
-            ++it;
-            const T *zin = V[j];
-            if (invd)
-              {
-                MPDG_CUDA(vec_scale<T>(z, V[j], invd, n, op->stream));
-                zin = z;
-              }
-            if (int e = apply<T>(op, (int)OutMode::Set, 1.0, V[j + 1], zin, nullptr, 1))
+            if (int e = apply<T>(op, (int)OutMode::Set, 1.0, V[jn + 1], invd ? z : V[jn], nullptr, 1))
               return e;
-            std::vector<const T *> Vc(V.begin(), V.begin() + j + 1);
-            MPDG_CUDA(vec_dots_against<T>(V[j + 1], Vc.data(), j + 1, n, d_h, red, op->stream));
-            MPDG_CUDA(vec_orth_update<T>(V[j + 1], Vc.data(), d_h, j + 1, n, d_h + j + 1, red, op->stream));
-            if (int e = fetch(j + 2))
-              return e;
-            const double hn = std::sqrt(std::max(0.0, op->h_scal[j + 1]));
-            for (int i = 0; i <= j; ++i)
-              H[i * m + j] = op->h_scal[i];
-            H[(j + 1) * m + j] = hn;
-            if (hn > 0.0)
-              MPDG_CUDA(vec_axpby<T>(V[j + 1], 1.0 / hn, V[j + 1], 0.0, nullptr, n, op->stream));
-            for (int i = 0; i < j; ++i)
+            std::vector<const T *> Vc(V.begin(), V.begin() + jn + 1);
+            MPDG_CUDA(vec_dots_against<T>(V[jn + 1], Vc.data(), jn + 1, n, d_h, red, op->stream));
+            MPDG_CUDA(vec_orth_update<T>(V[jn + 1], Vc.data(), d_h, jn + 1, n, d_h + jn + 1, red, op->stream));
+            MPDG_CUDA(cudaMemcpyAsync(op->h_scal + 32 * (jn & 1), d_h, sizeof(double) * (jn + 2), cudaMemcpyDeviceToHost,
+                                      op->stream));
+            MPDG_CUDA(cudaEventRecord(op->ev_gmres[jn & 1], op->stream));
+            if (jn + 1 < m)
+              MPDG_CUDA(gmres_next<T>(V[jn + 1], z, invd, d_h + jn + 1, n, op->stream));
+            if (jn > 0)
               {
-                const double t0 = H[i * m + j], t1 = H[(i + 1) * m + j];
-                H[i * m + j]       = cs[i] * t0 + sn[i] * t1;
-                H[(i + 1) * m + j] = -sn[i] * t0 + cs[i] * t1;
-              }
-            const double a = H[j * m + j], c = H[(j + 1) * m + j];
-            const double r = std::hypot(a, c);
-            cs[j]          = a / r;
-            sn[j]          = c / r;
-            H[j * m + j]       = r;
-            H[(j + 1) * m + j] = 0.0;
-            g[j + 1]           = -sn[j] * g[j];
-            g[j]               = cs[j] * g[j];
-            res                = std::abs(g[j + 1]);
-            hist.push_back(res);
-            state = ctl.check(it, res);
-            if (state != 0 || hn == 0.0)
-              {
-                ++j;
-                break;
+                if (int e = column(jn - 1))
+                  return e;
+                j = jn;
               }
           }
+        if (!stopped)
+          {
+            if (int e = column(m - 1))
+              return e;
+            j = m;
+          }
+        // a discarded column may still be on its way into the slots
+        MPDG_CUDA(cudaStreamSynchronize(op->stream));
         for (int i = j - 1; i >= 0; --i)
           {
             double s = g[i];
@@ -988,12 +1007,8 @@ namespace
           }
         std::memcpy(op->h_scal, y.data(), sizeof(double) * j);
         MPDG_CUDA(cudaMemcpyAsync(d_h, op->h_scal, sizeof(double) * j, cudaMemcpyHostToDevice, op->stream));
-        MPDG_CUDA(vec_fill<T>(z, T(0), n, op->stream));
         std::vector<const T *> Vc(V.begin(), V.begin() + j);
-        MPDG_CUDA(vec_multiaxpy<T>(z, Vc.data(), d_h, j, n, 1.0, op->stream));
-        if (invd)
-          MPDG_CUDA(vec_scale<T>(z, z, invd, n, op->stream));
-        MPDG_CUDA(vec_axpby<T>(x, 1.0, x, 1.0, z, n, op->stream));
+        MPDG_CUDA(gmres_update_x<T>(x, invd, Vc.data(), d_h, j, n, op->stream));
         MPDG_CUDA(cudaStreamSynchronize(op->stream));
         if (state != 0)
           break;
@@ -1183,6 +1198,9 @@ mpdg_op_destroy(mpdg_op *op)
   cudaFree(op->d_part);
   for (cudaEvent_t e : op->ev)
     cudaEventDestroy(e);
+  for (cudaEvent_t e : op->ev_gmres)
+    if (e)
+      cudaEventDestroy(e);
   if (op->s_h2d)
     cudaStreamDestroy(op->s_h2d);
   if (op->s_d2h)

@@ -257,13 +257,13 @@ namespace mpdg
   template <typename T>
   cudaError_t vec_dots_against(const T *w, const T *const *v, int m, long long n, double *out_dev, Reducer red,
                                cudaStream_t s);
-  // dst = src * invd (Jacobi)
+  // GMRES: x += invd (sum_k c_k v_k) (coefficients on the device, invd null: no preconditioner)
   template <typename T>
-  cudaError_t vec_scale(T *dst, const T *src, const T *invd, long long n, cudaStream_t s);
-  // x += sum_k c_k v_k (coefficients on the device), then optionally x *= invd first on the sum
+  cudaError_t gmres_update_x(T *x, const T *invd, const T *const *v, const double *coef_dev, int m, long long n,
+                             cudaStream_t s);
+  // GMRES: v /= sqrt(*norm2_dev), z = invd v (invd null: z untouched)
   template <typename T>
-  cudaError_t vec_multiaxpy(T *x, const T *const *v, const double *coef_dev, int m, long long n, double post_scale,
-                            cudaStream_t s);
+  cudaError_t gmres_next(T *v, T *z, const T *invd, const double *norm2_dev, long long n, cudaStream_t s);
   // w -= sum_k h_k v_k and returns ||w||^2 into out_dev (coefficients on the device)
   template <typename T>
   cudaError_t vec_orth_update(T *w, const T *const *v, const double *h_dev, int m, long long n, double *out_dev,

@@ -80,27 +80,20 @@ namespace mpdg
       __syncthreads();
       if (!last)
         return;
-      for (int k = 0; k < m_active; ++k)
+      // one warp per value: up to 33 values (GMRES) without a barrier between them
+      for (int k = warp; k < m_active; k += NWARP)
         {
           double s = MAX ? -INFINITY : 0.0;
-          for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+          for (int b = lane; b < (int)gridDim.x; b += 32)
             {
               const double p = __ldcg(red.partials + k * RED_BLOCKS + b);
               s              = MAX ? fmax(s, p) : s + p;
             }
           s = MAX ? warp_max(s) : warp_sum(s);
           if (lane == 0)
-            sh[0][warp] = s;
-          __syncthreads();
-          if (threadIdx.x == 0)
-            {
-              double t = sh[0][0];
-              for (int w = 1; w < NWARP; ++w)
-                t = MAX ? fmax(t, sh[0][w]) : t + sh[0][w];
-              tot[k] = t;
-            }
-          __syncthreads();
+            tot[k] = s;
         }
+      __syncthreads();
       if (threadIdx.x == 0)
         {
           fin(tot);
@@ -310,14 +303,6 @@ namespace mpdg
         x[i] += (double)e[i];
     }
 
-    template <typename T>
-    __global__ void
-    scale_kernel(T *d, const T *s, const T *w, long long n)
-    {
-      for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        d[i] = w ? s[i] * w[i] : s[i];
-    }
-
     constexpr int MAXV = 32;
     template <typename T>
     struct VecList
@@ -350,28 +335,96 @@ namespace mpdg
       });
     }
 
-    // x += post * sum_k c_k v_k   (post = scalar); coefficients read from the device
+    // GMRES solution update x += d (sum_k c_k v_k) (d = 1 without a preconditioner), coefficients read from the
+    // device; 16-byte packs when every vector is aligned
     template <typename T>
     __global__ void
-    multiaxpy_kernel(T *x, const __grid_constant__ VecList<T> L, const double *c, int m, long long n, double post)
+    gmres_update_x_kernel(T *x, const T *__restrict__ invd, const __grid_constant__ VecList<T> L, const double *c, int m,
+                          long long n, int packed)
     {
       __shared__ double cs[MAXV];
       if (threadIdx.x < MAXV)
         cs[threadIdx.x] = threadIdx.x < m ? c[threadIdx.x] : 0.0;
       __syncthreads();
-      for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+      const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+      using P               = Pack<T>;
+      using V               = typename P::V;
+      const long long nv    = packed ? n / P::W : 0;
+      for (long long i = tid; i < nv; i += stride)
+        {
+          double s[P::W] = {};
+#pragma unroll 8
+          for (int k = 0; k < m; ++k)
+            {
+              V vv = reinterpret_cast<const V *>(L.v[k])[i];
+#pragma unroll
+              for (int e = 0; e < P::W; ++e)
+                s[e] += cs[k] * (double)P::at(vv, e);
+            }
+          V xv = reinterpret_cast<const V *>(x)[i];
+          V dv = xv;
+          if (invd)
+            dv = reinterpret_cast<const V *>(invd)[i];
+#pragma unroll
+          for (int e = 0; e < P::W; ++e)
+            P::at(xv, e) += invd ? (T)s[e] * P::at(dv, e) : (T)s[e];
+          reinterpret_cast<V *>(x)[i] = xv;
+        }
+      for (long long i = nv * P::W + tid; i < n; i += stride)
         {
           double s = 0.0;
           for (int k = 0; k < m; ++k)
             s += cs[k] * (double)L.v[k][i];
-          x[i] += (T)(post * s);
+          x[i] += invd ? (T)s * invd[i] : (T)s;
         }
     }
 
-    // h_k = w . v_k (k < m), plus ||w||^2 as entry m
-    // h_k = w . v_k (k < m <= MB), out[m] = |w|^2; 16-byte packs when every vector is aligned
-    template <typename T, int MB>
+    // Next basis vector v /= |v| (|v|^2 on the device) and its preconditioned copy z = d v, in one pass
+    template <typename T>
     __global__ void
+    gmres_next_kernel(T *v, T *z, const T *__restrict__ invd, const double *norm2, long long n, int packed)
+    {
+      const T         a   = (T)(1.0 / sqrt(*norm2));
+      const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+      using P               = Pack<T>;
+      using V               = typename P::V;
+      const long long nv    = packed ? n / P::W : 0;
+      for (long long i = tid; i < nv; i += stride)
+        {
+          V vv = reinterpret_cast<const V *>(v)[i];
+          V dv = vv;
+          if (invd)
+            dv = reinterpret_cast<const V *>(invd)[i];
+#pragma unroll
+          for (int e = 0; e < P::W; ++e)
+            {
+              P::at(vv, e) *= a;
+              P::at(dv, e) *= P::at(vv, e);
+            }
+          reinterpret_cast<V *>(v)[i] = vv;
+          if (invd)
+            reinterpret_cast<V *>(z)[i] = dv;
+        }
+      for (long long i = nv * P::W + tid; i < n; i += stride)
+        {
+          const T t = a * v[i];
+          v[i]      = t;
+          if (invd)
+            z[i] = invd[i] * t;
+        }
+    }
+
+    // Blocks per SM of the Gram-Schmidt kernels at basis size MB; the grid is that many blocks on every SM, all
+    // resident (at 592 blocks the kernels of 24 vectors, three to an SM, ran a second wave a third full: 161 us
+    // against 77 us for 20 vectors)
+    constexpr int gs_blocks(int mb) { return mb <= 8 ? 4 : (mb <= 16 ? 3 : 2); }
+
+    // h_k = w . v_k (k < m <= MB), out[m] = |w|^2; 16-byte packs when every vector is aligned.  The list is padded
+    // to MB with its first vector (whose lines are in L1), so that the MB loads of a step have no branch between
+    // them and are in flight together (30 vectors of 2.1 M doubles: 203 us with a test per vector and a
+    // barrier pair per value in the final sum, against 78 us for their bytes).
+    template <typename T, int MB>
+    __global__ void __launch_bounds__(RED_THREADS, gs_blocks(MB))
     dots_against_kernel(const T *w, const __grid_constant__ VecList<T> L, int m, long long n, double *out, Reducer red,
                         int packed)
     {
@@ -392,13 +445,12 @@ namespace mpdg
             }
 #pragma unroll
           for (int k = 0; k < MB; ++k)
-            if (k < m)
-              {
-                V vv = reinterpret_cast<const V *>(L.v[k])[i];
+            {
+              V vv = reinterpret_cast<const V *>(L.v[k])[i];
 #pragma unroll
-                for (int e = 0; e < P::W; ++e)
-                  a[k] += wd[e] * (double)P::at(vv, e);
-              }
+              for (int e = 0; e < P::W; ++e)
+                a[k] += wd[e] * (double)P::at(vv, e);
+            }
         }
       for (long long i = nv * P::W + tid; i < n; i += stride)
         {
@@ -420,9 +472,11 @@ namespace mpdg
       });
     }
 
-    // w -= sum_k h_k v_k (k < m <= MB); out[0] = ||w||^2
+    // w -= sum_k h_k v_k (k < m <= MB); out[0] = ||w||^2.  Walks from the high end of the vectors down: the dot
+    // products before it end there, and L2 still holds the last of what they read of every basis vector (and
+    // the next iteration's dot products start at the low end, where this pass ends).
     template <typename T, int MB>
-    __global__ void
+    __global__ void __launch_bounds__(RED_THREADS, gs_blocks(MB))
     orth_update_kernel(T *w, const __grid_constant__ VecList<T> L, const double *h, int m, long long n, double *out,
                        Reducer red, int packed)
     {
@@ -435,8 +489,9 @@ namespace mpdg
       using P               = Pack<T>;
       using V               = typename P::V;
       const long long nv    = packed ? n / P::W : 0;
-      for (long long i = tid; i < nv; i += stride)
+      for (long long i0 = tid; i0 < nv; i0 += stride)
         {
+          const long long i = nv - 1 - i0;
           V      wv = reinterpret_cast<const V *>(w)[i];
           double sd[P::W];
 #pragma unroll
@@ -444,13 +499,12 @@ namespace mpdg
             sd[e] = (double)P::at(wv, e);
 #pragma unroll
           for (int k = 0; k < MB; ++k)
-            if (k < m)
-              {
-                V vv = reinterpret_cast<const V *>(L.v[k])[i];
+            {
+              V vv = reinterpret_cast<const V *>(L.v[k])[i];
 #pragma unroll
-                for (int e = 0; e < P::W; ++e)
-                  sd[e] -= hs[k] * (double)P::at(vv, e);
-              }
+              for (int e = 0; e < P::W; ++e)
+                sd[e] -= hs[k] * (double)P::at(vv, e); // hs is 0 on the padding
+            }
 #pragma unroll
           for (int e = 0; e < P::W; ++e)
             {
@@ -631,21 +685,26 @@ namespace mpdg
   }
   template <typename T>
   cudaError_t
-  vec_scale(T *d, const T *src, const T *w, long long n, cudaStream_t s)
-  {
-    scale_kernel<T><<<stream_blocks(n), 256, 0, s>>>(d, src, w, n);
-    return cudaGetLastError();
-  }
-  template <typename T>
-  cudaError_t
-  vec_multiaxpy(T *x, const T *const *v, const double *c, int m, long long n, double post, cudaStream_t s)
+  gmres_update_x(T *x, const T *invd, const T *const *v, const double *c, int m, long long n, cudaStream_t s)
   {
     if (m < 1 || m > MAXV)
       return cudaErrorInvalidValue;
     VecList<T> L{};
+    int        packed = aligned16(x) && aligned16(invd);
     for (int k = 0; k < m; ++k)
-      L.v[k] = v[k];
-    multiaxpy_kernel<T><<<stream_blocks(n), 256, 0, s>>>(x, L, c, m, n, post);
+      {
+        L.v[k] = v[k];
+        packed = packed && aligned16(v[k]);
+      }
+    gmres_update_x_kernel<T><<<stream_blocks(packed ? (n + 3) / 4 : n), 256, 0, s>>>(x, invd, L, c, m, n, packed);
+    return cudaGetLastError();
+  }
+  template <typename T>
+  cudaError_t
+  gmres_next(T *v, T *z, const T *invd, const double *norm2, long long n, cudaStream_t s)
+  {
+    const int packed = aligned16(v) && aligned16(z) && aligned16(invd);
+    gmres_next_kernel<T><<<stream_blocks(packed ? (n + 3) / 4 : n), 256, 0, s>>>(v, z, invd, norm2, n, packed);
     return cudaGetLastError();
   }
   template <typename T>
@@ -661,14 +720,20 @@ namespace mpdg
         L.v[k] = v[k];
         packed = packed && aligned16(v[k]);
       }
-    if (m <= 4)
-      dots_against_kernel<T, 4><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed);
-    else if (m <= 8)
-      dots_against_kernel<T, 8><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed);
-    else if (m <= 16)
-      dots_against_kernel<T, 16><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed);
-    else
-      dots_against_kernel<T, MAXV><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed);
+    const int mb = (m + 3) / 4 * 4;
+    for (int k = m; k < mb; ++k)
+      L.v[k] = v[0];
+    switch (mb)
+      {
+        case 4: dots_against_kernel<T, 4><<<148 * gs_blocks(4), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 8: dots_against_kernel<T, 8><<<148 * gs_blocks(8), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 12: dots_against_kernel<T, 12><<<148 * gs_blocks(12), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 16: dots_against_kernel<T, 16><<<148 * gs_blocks(16), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 20: dots_against_kernel<T, 20><<<148 * gs_blocks(20), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 24: dots_against_kernel<T, 24><<<148 * gs_blocks(24), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        case 28: dots_against_kernel<T, 28><<<148 * gs_blocks(28), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed); break;
+        default: dots_against_kernel<T, MAXV><<<148 * gs_blocks(MAXV), RED_THREADS, 0, s>>>(w, L, m, n, out, red, packed);
+      }
     return cudaGetLastError();
   }
   template <typename T>
@@ -685,14 +750,20 @@ namespace mpdg
         L.v[k] = v[k];
         packed = packed && aligned16(v[k]);
       }
-    if (m <= 4)
-      orth_update_kernel<T, 4><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed);
-    else if (m <= 8)
-      orth_update_kernel<T, 8><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed);
-    else if (m <= 16)
-      orth_update_kernel<T, 16><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed);
-    else
-      orth_update_kernel<T, MAXV><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed);
+    const int mb = (m + 3) / 4 * 4;
+    for (int k = m; k < mb; ++k)
+      L.v[k] = v[0];
+    switch (mb)
+      {
+        case 4: orth_update_kernel<T, 4><<<148 * gs_blocks(4), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 8: orth_update_kernel<T, 8><<<148 * gs_blocks(8), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 12: orth_update_kernel<T, 12><<<148 * gs_blocks(12), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 16: orth_update_kernel<T, 16><<<148 * gs_blocks(16), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 20: orth_update_kernel<T, 20><<<148 * gs_blocks(20), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 24: orth_update_kernel<T, 24><<<148 * gs_blocks(24), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        case 28: orth_update_kernel<T, 28><<<148 * gs_blocks(28), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed); break;
+        default: orth_update_kernel<T, MAXV><<<148 * gs_blocks(MAXV), RED_THREADS, 0, s>>>(w, L, h, m, n, out, red, packed);
+      }
     return cudaGetLastError();
   }
   template <typename T>
@@ -807,9 +878,9 @@ namespace mpdg
   template cudaError_t vec_axpby<T>(T *, double, const T *, double, const T *, long long, cudaStream_t);        \
   template cudaError_t vec_multidot<T>(const T *const *, const T *const *, int, long long, double *, Reducer,    \
                                        cudaStream_t);                                                           \
-  template cudaError_t vec_scale<T>(T *, const T *, const T *, long long, cudaStream_t);                        \
-  template cudaError_t vec_multiaxpy<T>(T *, const T *const *, const double *, int, long long, double,          \
-                                        cudaStream_t);                                                          \
+  template cudaError_t gmres_update_x<T>(T *, const T *, const T *const *, const double *, int, long long,       \
+                                         cudaStream_t);                                                         \
+  template cudaError_t gmres_next<T>(T *, T *, const T *, const double *, long long, cudaStream_t);             \
   template cudaError_t vec_dots_against<T>(const T *, const T *const *, int, long long, double *, Reducer,       \
                                            cudaStream_t);                                                       \
   template cudaError_t vec_orth_update<T>(T *, const T *const *, const double *, int, long long, double *,      \
