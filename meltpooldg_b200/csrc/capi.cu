@@ -1820,17 +1820,33 @@ mpdg_op_create_rhs(mpdg_op *op, double *dst, const double *a, const double *b, c
   if (op->kind == MPDG_HEAT)
     {
       // v = (rho c_p/dt)(T_old - T) + q ; dst += M v - K_k T   (plain reads, free rows)
-      double *v = op->vec<double>("rhs_tmp");
-      if (!v)
-        return fail(MPDG_ERR_NOMEM, "rhs work vector");
       const double s = op->rho_cp / op->dt;
-      MPDG_CUDA(vec_axpby<double>(v, -s, a, b ? s : 0.0, b, op->ndofs, op->stream));
-      if (c)
-        MPDG_CUDA(vec_axpby<double>(v, 1.0, v, 1.0, c, op->ndofs, op->stream));
-      if (int e = apply<double>(op, (int)OutMode::Add, 1.0, dst, v, nullptr, 0, 1))
-        return e;
-      if (int e = apply<double>(op, (int)OutMode::Add, -1.0, dst, a, nullptr, 0, 2))
-        return e;
+      if (op->degree <= 2 && !op->d_mask && !op->banded())
+        {
+          HeatLaunch<double> h;
+          h.degree = op->degree;
+          h.geo    = heat_geom(op, 1.0);
+          h.grid   = op->grid();
+          h.sync   = op->sync();
+          h.kconst = op->k;
+          h.kcell  = op->d_k64;
+          h.src    = a;
+          h.dst    = dst;
+          MPDG_CUDA(heat_rhs(h, s, b, c, op->stream));
+        }
+      else
+        {
+          double *v = op->vec<double>("rhs_tmp");
+          if (!v)
+            return fail(MPDG_ERR_NOMEM, "rhs work vector");
+          MPDG_CUDA(vec_axpby<double>(v, -s, a, b ? s : 0.0, b, op->ndofs, op->stream));
+          if (c)
+            MPDG_CUDA(vec_axpby<double>(v, 1.0, v, 1.0, c, op->ndofs, op->stream));
+          if (int e = apply<double>(op, (int)OutMode::Add, 1.0, dst, v, nullptr, 0, 1))
+            return e;
+          if (int e = apply<double>(op, (int)OutMode::Add, -1.0, dst, a, nullptr, 0, 2))
+            return e;
+        }
       if (op->d_vfield[0])
         {
           // dst -= int rho c_p (v . grad T) phi (heat_diffuse_operator.cpp:499-500), plain reads

@@ -359,6 +359,103 @@ namespace mpdg
     }
   };
 
+  // ---- k <= 2: the constant-material right-hand side in one pass, dst += M v - K_k T with
+  // v = (rho c_p / dt) (T_old - T) + q (plain reads): both inputs go to the eigenbasis, one result comes back
+  template <int K>
+  struct HeatRhsArgs
+  {
+    HeatArgs<double, K + 1> a;    // alpha: h_x h_y h_z, kscale 1, src: T
+    double                  rate; // rho c_p / dt
+    const double           *temp_old, *q; // may be null
+  };
+
+  template <int K>
+  struct HeatRhsCellOp
+  {
+    static constexpr int  N = K + 1, NE = (N + 1) / 2, NO = N / 2;
+    static constexpr bool NODES = false;
+    const HeatRhsArgs<K> &r;
+    struct Cell
+    {
+      double    k;
+      long long first; // the cell's first lattice point (a lane outside the mesh: the nearest cell's)
+    };
+    __device__ __forceinline__ Cell
+    load(bool, int cx, int cy, int cz) const
+    {
+      const GridDesc &g = r.a.g;
+      const int       x = min(cx, g.m[0] - 1), y = min(cy, g.m[1] - 1);
+      return Cell{r.a.kcell ? r.a.kcell[(long long)x + (long long)g.m[0] * ((long long)y + (long long)g.m[1] * cz)] : r.a.kconst,
+                  K * x + (long long)g.n[0] * (K * y + (long long)g.n[1] * (K * cz))};
+    }
+    template <bool DOT>
+    __device__ __forceinline__ double
+    apply(double *u, const Cell &c) const
+    {
+      const HeatArgs<double, N> &a  = r.a;
+      const int                  sy = a.g.n[0], sz = a.g.n[0] * a.g.n[1];
+      double                     v[N * N * N];
+#pragma unroll
+      for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            {
+              const int       n = (l * N + j) * N + i;
+              const long long p = c.first + (j * sy + l * sz + i);
+              double          x = -r.rate * u[n];
+              if (r.temp_old)
+                x = fma(r.rate, __ldg(r.temp_old + p), x);
+              if (r.q)
+                x += __ldg(r.q + p);
+              v[n] = x;
+            }
+      const double *tb = fd_table<double>(K), *we = tb, *wo = tb + NE * NE, *lam = tb + NE * NE + NO * NO;
+      xy_planes<double, N, N, true>(u, we, wo);
+      xy_planes<double, N, N, true>(v, we, wo);
+#pragma unroll
+      for (int q = 0; q < N * N; ++q)
+        {
+          fwd_line<double, N, N * N>(u, q, we, wo);
+          fwd_line<double, N, N * N>(v, q, we, wo);
+        }
+      const double kx = -c.k * a.cx, ky = -c.k * a.cy, kz = -c.k * a.cz;
+#pragma unroll
+      for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int b = 0; b < N; ++b)
+          {
+            const double tyz = fma(ky, lam[b], kz * lam[l]);
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+              {
+                const int n = (l * N + b) * N + i;
+                u[n]        = fma(fma(kx, lam[i], tyz), u[n], a.alpha * v[n]);
+              }
+          }
+#pragma unroll
+      for (int q = 0; q < N * N; ++q)
+        bwd_line<double, N, N * N>(u, q, we, wo);
+      xy_planes<double, N, N, false>(u, we, wo);
+      return 0.0;
+    }
+  };
+
+  constexpr int heat_rhs_minb(int K) { return K == 1 ? 6 : 3; }
+
+  template <int K>
+  __global__ void __launch_bounds__(MARCH_NT, heat_rhs_minb(K))
+  heat_rhs_kernel(const __grid_constant__ HeatRhsArgs<K> r)
+  {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned                        s_ticket;
+    __shared__ __align__(8) unsigned long long s_bars[2];
+    HeatRhsCellOp<K>                           op{r};
+    march_body<K, double, OutMode::Add, HeatRhsCellOp<K>>(r.a.g, r.a.s, r.a.src, r.a.dst, nullptr, false, op,
+                                                          reinterpret_cast<double *>(smem_raw), &s_ticket, s_bars);
+  }
+
 #ifndef MPDG_MARCH_MINB_F64
 #define MPDG_MARCH_MINB_F64 4
 #endif
@@ -664,6 +761,48 @@ namespace mpdg
         kern<<<nbricks, L::BR::NT, L::bytes, stream>>>(a);
       }
     return cudaGetLastError();
+  }
+
+  template <int K>
+  static cudaError_t
+  launch_heat_rhs(const HeatLaunch<double> &h, double rate, const double *temp_old, const double *q, cudaStream_t stream)
+  {
+    cudaError_t e = upload_fd_tables();
+    if (e != cudaSuccess)
+      return e;
+    HeatRhsArgs<K> r{};
+    r.a.cx     = h.geo.cx;
+    r.a.cy     = h.geo.cy;
+    r.a.cz     = h.geo.cz;
+    r.a.g      = h.grid;
+    r.a.s      = h.sync;
+    r.a.alpha  = h.geo.mass_coef;
+    r.a.kconst = h.kconst;
+    r.a.kcell  = h.kcell;
+    r.a.src    = h.src;
+    r.a.dst    = h.dst;
+    r.rate     = rate;
+    r.temp_old = temp_old;
+    r.q        = q;
+    static std::atomic<unsigned long long> devices{0};
+    auto                                   kern  = heat_rhs_kernel<K>;
+    constexpr size_t                       bytes = MarchLayout<K, double>::bytes;
+    if ((e = ensure_smem(kern, bytes, devices)) != cudaSuccess)
+      return e;
+    const unsigned ctas = march_grid(r.a.g, MarchShape<K, double>::BZ, heat_rhs_minb(K));
+    kern<<<ctas, MARCH_NT, bytes, stream>>>(r);
+    return cudaGetLastError();
+  }
+
+  cudaError_t
+  heat_rhs(const HeatLaunch<double> &h, double rate, const double *temp_old, const double *q, cudaStream_t s)
+  {
+    switch (h.degree)
+      {
+        case 1: return launch_heat_rhs<1>(h, rate, temp_old, q, s);
+        case 2: return launch_heat_rhs<2>(h, rate, temp_old, q, s);
+        default: return cudaErrorInvalidValue;
+      }
   }
 
   template <typename T>

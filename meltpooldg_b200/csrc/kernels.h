@@ -43,6 +43,10 @@ namespace mpdg
   template <typename T>
   cudaError_t heat_apply(const HeatLaunch<T> &h, cudaStream_t s);
 
+  // dst += M v - K_k src on the free rows, v = rate (temp_old - src) + q (k <= 2, no per-DoF mask; plain reads;
+  // temp_old and q may be null); h: degree, geo (mass_coef: the cell volume), grid, sync, kconst, kcell, src, dst
+  cudaError_t heat_rhs(const HeatLaunch<double> &h, double rate, const double *temp_old, const double *q, cudaStream_t s);
+
   template <typename T>
   cudaError_t heat_diagonal(const GridDesc &g, int K, const HeatGeom &geo, double kconst, const T *kcell,
                             T *diag, bool invert, double threshold, cudaStream_t s);
