@@ -47,7 +47,8 @@ namespace mpdg
     const uint8_t *cmask;  // optional per-DoF Dirichlet flags (device), may be null
     unsigned       acc_lo_z = 0; // the lattice is a z-slab of a larger one: its low z plane already
                                  // holds the previous slab's contributions and is only added into
-    int            bz = 0;       // cell layers per segment of the column-marching apply (march.cuh)
+    int            bz = 0;       // cell layers per segment of the column-marching apply (march.cuh); for
+                                 // bricks: < 0 cuts z into nbr[2] nearly equal parts, else BZ layers each
   };
 
   constexpr unsigned SPIN_LIMIT    = 1u << 22; // x 32 ns sleeps: ~0.1-0.2 s
@@ -181,6 +182,8 @@ namespace mpdg
     static constexpr int RSTEP  = NT / PX;
     static constexpr int RITER  = RSTEP > 0 ? (ROWS + RSTEP - 1) / RSTEP : 0;
     int            c0[3];                // first cell of the brick
+    int            b[3];                 // brick index
+    int            layers;               // cell layers in z (BZ, or the brick's part)
     int            g0[3];                // first lattice point (K c0)
     int            nv[3];                // lattice points of the brick inside the domain
     int            lo_sh[3], hi_sh[3];   // low / high face shared with a neighbour brick
@@ -194,10 +197,15 @@ namespace mpdg
     set(const GridDesc &g, unsigned t)
     {
       id    = t;
-      c0[0] = (int)(t % (unsigned)g.nbr[0]) * BX;
-      c0[1] = (int)((t / (unsigned)g.nbr[0]) % (unsigned)g.nbr[1]) * BY;
-      c0[2] = (int)(t / (unsigned)(g.nbr[0] * g.nbr[1])) * BZ;
-      const int B[3] = {BX, BY, BZ}, P[3] = {PX, PY, PZ};
+      b[0]  = (int)(t % (unsigned)g.nbr[0]);
+      b[1]  = (int)((t / (unsigned)g.nbr[0]) % (unsigned)g.nbr[1]);
+      b[2]  = (int)(t / (unsigned)(g.nbr[0] * g.nbr[1]));
+      c0[0] = b[0] * BX;
+      c0[1] = b[1] * BY;
+      const bool even_z = g.bz < 0;
+      c0[2]  = even_z ? (int)((long long)g.m[2] * b[2] / g.nbr[2]) : b[2] * BZ;
+      layers = (even_z ? (int)((long long)g.m[2] * (b[2] + 1) / g.nbr[2]) : min(c0[2] + BZ, g.m[2])) - c0[2];
+      const int B[3] = {BX, BY, even_z ? layers : BZ}, P[3] = {PX, PY, K * B[2] + 1};
       any_con        = g.cmask != nullptr;
 #pragma unroll
       for (int d = 0; d < 3; ++d)
@@ -354,7 +362,7 @@ namespace mpdg
         if (side == 0 && br.lo_sh[0])
           continue;
         const int px = side ? br.nv[0] - 1 : 0;
-        for (int e = threadIdx.x; e < BR::PY * BR::PZ; e += BR::NT)
+        for (int e = threadIdx.x; e < BR::PY * br.nv[2]; e += BR::NT)
           {
             const int py = e % BR::PY, pz = e / BR::PY;
             if (py < br.nv[1] && pz < br.nv[2])
@@ -367,7 +375,7 @@ namespace mpdg
         if (side == 0 && br.lo_sh[1])
           continue;
         const int py = side ? br.nv[1] - 1 : 0;
-        for (int e = threadIdx.x; e < BR::PX * BR::PZ; e += BR::NT)
+        for (int e = threadIdx.x; e < BR::PX * br.nv[2]; e += BR::NT)
           {
             const int px = e % BR::PX, pz = e / BR::PX;
             if (px < br.nv[0] && pz < br.nv[2])
@@ -507,7 +515,7 @@ namespace mpdg
       {
         const unsigned t  = threadIdx.x + 1; // offsets (ox,oy,oz) in {0,1}^3 minus (0,0,0)
         const int      ox = (t & 1u) ? 1 : 0, oy = (t & 2u) ? 1 : 0, oz = (t & 4u) ? 1 : 0;
-        const int bx = br.c0[0] / BR::BX - ox, by = br.c0[1] / BR::BY - oy, bz = br.c0[2] / BR::BZ - oz;
+        const int bx = br.b[0] - ox, by = br.b[1] - oy, bz = br.b[2] - oz;
         if (bx >= 0 && by >= 0 && bz >= 0)
           {
             const unsigned nb = (unsigned)bx + (unsigned)g.nbr[0] * ((unsigned)by + (unsigned)g.nbr[1] * (unsigned)bz);

@@ -727,11 +727,13 @@ namespace mpdg
           kern<<<nbricks, MARCH_NT, ML::bytes, stream>>>(a);
           return cudaGetLastError();
         }
-    const unsigned nbricks = (unsigned)h.grid.nbr[0] * h.grid.nbr[1] * h.grid.nbr[2];
     if constexpr (K >= 3)
       if (h.grid.cmask == nullptr && h.march)
         {
           using PL = PencilLayout<K, T>;
+          a.g.nbr[2] = pencil_plan(a.g.m, PencilShape<K>::BX, PencilShape<K>::BY, PencilShape<K>::BZ, 148 * PencilShape<K>::MINB);
+          a.g.bz     = -1;
+          const unsigned nbricks = (unsigned)a.g.nbr[0] * a.g.nbr[1] * a.g.nbr[2];
           static std::atomic<unsigned long long> dev_plain{0}, dev_dot{0};
           if constexpr (MODE == OutMode::Set)
             if (h.dot.part != nullptr)
@@ -753,7 +755,8 @@ namespace mpdg
     if (h.dot.part != nullptr)
       return cudaErrorInvalidValue; // the brick kernel has no fused dot (heat_apply_fuses_dot is false)
     {
-        auto                                   kern = heat_apply_kernel<K, T, MODE>;
+        const unsigned nbricks = (unsigned)h.grid.nbr[0] * h.grid.nbr[1] * h.grid.nbr[2];
+        auto           kern    = heat_apply_kernel<K, T, MODE>;
         static std::atomic<unsigned long long> dev_brick{0};
         cudaError_t                            e = ensure_smem(kern, L::bytes, dev_brick);
         if (e != cudaSuccess)
@@ -859,7 +862,7 @@ namespace mpdg
           nb *= (m[d] + sh[d] - 1) / sh[d];
         most = std::max(most, nb);
       }
-    return most;
+    return march ? std::max(most, PENCIL_MIN_FLAGS) : most;
   }
 
   template <int K, typename T>

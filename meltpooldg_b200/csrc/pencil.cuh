@@ -48,8 +48,13 @@
 #define MPDG_PENCIL_PREFETCH -1 // -1: by degree and precision (measured); 0 off; 1 on
 #endif
 
+#include <algorithm>
+
 namespace mpdg
 {
+  // bricks of any mesh: at most the full-height ones or this many (brick flags, dot partials)
+  constexpr long long PENCIL_MIN_FLAGS = 8192;
+
   template <int K>
   struct PencilShape
   {
@@ -76,6 +81,30 @@ namespace mpdg
     using BR = Brick<K, S::BX, S::BY, S::BZ, S::NT>;
   };
 
+  // Parts of z for a mesh: the number of nearly equal parts whose bricks take the least time on the
+  // resident slots (the cost model of march_plan), or the full-height bricks where that gains less than
+  // 15 % by the model.  Measured at 64^3: FE_Q(3) FP64 16 parts 78.8 us (1024 bricks on 740 slots), 11 parts
+  // one wave, 72 us; FE_Q(4) FP64 16 parts 120.6, 9 parts (one wave, 12 % by the model) 121.8.  Small meshes
+  // gain the most: full-height bricks leave most slots without one.
+  inline int
+  pencil_plan(const int m[3], int bx, int by, int bz_full, int slots)
+  {
+    const long long cols = (long long)((m[0] + bx - 1) / bx) * ((m[1] + by - 1) / by);
+    const int       whole = (m[2] + bz_full - 1) / bz_full;
+    const long long cap  = std::max(cols * whole, PENCIL_MIN_FLAGS);
+    auto            cost = [&](int n) {
+      const double    b    = (double)m[2] / n;
+      const long long nb   = cols * n, full = nb / slots;
+      const double    part = (double)(nb % slots) / slots;
+      return (b + 1.0) * (double)full + (part > 0.0 ? (b + 2.0) * (0.57 + 0.43 * part) : 0.0);
+    };
+    int nseg = whole;
+    for (int n = std::max(1, (m[2] + 15) / 16); n <= m[2] && cols * n <= cap; ++n)
+      if (cost(n) < cost(nseg))
+        nseg = n;
+    return cost(nseg) < 0.85 * cost(whole) ? nseg : whole;
+  }
+
   // Op supplies the fast-diagonalisation tables and the per-cell scaling:
   //   we(), wo(), lam()  1-D tables;  alpha(), cxg(), cyg(), czg()  geometry;  kcell(cell)  k_c.
   // With DOT the x lines also add d_mode * (modal value)^2, i.e. the cells' forms src_c^T A_c src_c,
@@ -97,8 +126,7 @@ namespace mpdg
     constexpr bool PF = MPDG_PENCIL_PREFETCH < 0 ? (K == 3 || sizeof(T) == 4) : MPDG_PENCIL_PREFETCH != 0;
     if (!brick_begin<BR, T, MODE>(br, g, s, dst, bvec, s_ticket))
       return;
-    const int ncx = min(BX, g.m[0] - br.c0[0]), ncy = min(SH::BY, g.m[1] - br.c0[1]),
-              ncz = min(SH::BZ, g.m[2] - br.c0[2]);
+    const int ncx = min(BX, g.m[0] - br.c0[0]), ncy = min(SH::BY, g.m[1] - br.c0[1]), ncz = br.layers;
     const int  plast = K * ncx;               // brick's high x face (x point)
     const bool xin   = p <= plast;
     const int  sy = br.sy, sz = br.sz;

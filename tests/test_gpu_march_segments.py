@@ -41,3 +41,42 @@ def test_march_modes_and_offsets(degree, m, offset):
     g.residual(r, placed(b, torch.float64), placed(x, torch.float64))
     assert rel_err(r.cpu().numpy(), b - ref) <= 1e-12
     assert g.device_errors() == 0
+
+
+@pytest.mark.parametrize("degree", [3, 4])
+@pytest.mark.parametrize("m", [(1, 1, 1), (5, 6, 9), (33, 3, 5), (64, 2, 17), (32, 1, 40)])
+def test_pencil_parts(degree, m):
+    """Pencil apply on meshes whose z direction is cut into few, many and unequal parts."""
+    import torch
+
+    o, g, om, cm = heat_pair(degree, m, faces=0b100110, length=(1.1, 0.9, 1.3))
+    x, b = uniform_dofs(om, seed=6), uniform_dofs(om, seed=7)
+    ref = o.vmult(x)
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 2e-6)):
+        y = torch.full((om.ndofs,), float("nan"), dtype=dt, device="cuda")
+        g.vmult(y, to_gpu(x, dt))
+        assert rel_err(y.cpu().numpy(), ref) <= tol
+    y = to_gpu(b)
+    g.vmult_add(y, to_gpu(x), 2.0)
+    assert rel_err(y.cpu().numpy(), b + 2.0 * np.where(cm == 0, ref, 0.0)) <= 1e-12
+    assert g.device_errors() == 0
+
+
+@pytest.mark.parametrize("degree", [1, 2])
+@pytest.mark.parametrize("m", [(1, 2, 1), (33, 5, 3), (40, 9, 11)])
+@pytest.mark.parametrize("parts", ["all", "no_q", "no_old", "only_T"])
+def test_rhs_in_one_pass(degree, m, parts):
+    """create_rhs accumulates M (rho c_p / dt (T_old - T) + q) - K T, for each optional input left out."""
+    o, g, om, cm = heat_pair(degree, m, faces=0b010100, length=(1.1, 0.9, 1.3))
+    T, old, q, dst = (uniform_dofs(om, seed=s) for s in (1, 2, 3, 4))
+    old = None if parts in ("no_old", "only_T") else old
+    q = None if parts in ("no_q", "only_T") else q
+    y = to_gpu(dst)
+    g.create_rhs(y, to_gpu(T), None if old is None else to_gpu(old), None if q is None else to_gpu(q))
+    zero = np.zeros(om.ndofs)
+    # T_old left out drops its term (not the one of T), as a zero vector does
+    ref = dst.copy()
+    o.create_rhs(ref, T, zero if old is None else old, zero if q is None else q)
+    # sums of two products of 27 terms with coefficients up to rho c_p / dt = 130
+    assert rel_err(y.cpu().numpy(), ref) <= 1e-12
+    assert g.device_errors() == 0
