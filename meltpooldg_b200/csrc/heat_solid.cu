@@ -1,4 +1,4 @@
-// Heat operator with temperature-dependent material (solid / liquid phases), FE_Q(1, 2).
+// Heat operator with temperature-dependent material (solid / liquid phases), FE_Q(1..3).
 //
 // Reference: source/heat/heat_diffuse_operator.cpp, tangent_local_cell_operation :1029-1050 with
 // do_solidification (material of Material::compute_parameters, MaterialTypes::liquid_solid,
@@ -353,7 +353,8 @@ namespace mpdg
 #ifndef MPDG_SOLID_MINB
 #define MPDG_SOLID_MINB 0
 #endif
-    // CTAs (of 128 threads) per SM the register allocation is held to
+    // CTAs (of 128 threads) per SM the register allocation is held to; residual, diagonal and tangent, 64^3 FE_Q(2) FP64:
+    // 490 us at 3, 576 at 2, 590 at 4 (1007 before)
     template <int K, typename T>
     struct SolidMinBlocks
     {

@@ -20,8 +20,9 @@
 // elements in between, (address / sizeof(T)) mod (16 / sizeof(T)), which every reader computes from the
 // row's index.  Granules that would reach outside the vector (its first and last row only) are fetched
 // point by point.  Against per-element copies (cp.async of all K + 1 planes by every thread, with the
-// row and bounds arithmetic of each point) this took the FE_Q(2) FP64 apply from 1439 to about 1000 warp
-// instructions per 32 cells; the kernel is bound by instruction issue and latency, not by bandwidth.
+// row and bounds arithmetic of each point) this took the FE_Q(2) FP64 apply from 1439 to about 1100 warp
+// instructions per 32 cells (96^3: 93.7 -> 60.2 us, FP32 128^3: 141 -> 96 us); the kernel is bound by
+// instruction issue and latency, not by bandwidth.
 //
 // Segment length.  bz is chosen per mesh by march_plan (below).
 #pragma once

@@ -422,7 +422,7 @@ namespace mpdg
     // h_k = w . v_k (k < m <= MB), out[m] = |w|^2; 16-byte packs when every vector is aligned.  The list is padded
     // to MB with its first vector (whose lines are in L1), so that the MB loads of a step have no branch between
     // them and are in flight together (30 vectors of 2.1 M doubles: 203 us with a test per vector and a
-    // barrier pair per value in the final sum, against 78 us for their bytes).
+    // barrier pair per value in the final sum, 97 us now, 78 us for their bytes).
     template <typename T, int MB>
     __global__ void __launch_bounds__(RED_THREADS, gs_blocks(MB))
     dots_against_kernel(const T *w, const __grid_constant__ VecList<T> L, int m, long long n, double *out, Reducer red,
