@@ -217,7 +217,7 @@ namespace mpdg
 #pragma unroll(K == 1 ? 2 : 1)
         for (int qz = 0; qz < N; ++qz)
           {
-            const T *bz = a.t.B + qz * N, *gz = a.t.Gz + qz * (N - 1);
+            const T *bz = a.t.B + qz * N, *gz = a.t.G[2] + qz * (N - 1);
             T        t[N2], tz[N2], S[N2], k[N2], F[N2];
             solid_plane<T, N>(a, c, bz, gz, t, tz, S);
             if constexpr (RHS)
@@ -236,7 +236,8 @@ namespace mpdg
             else
               {
                 T u[N2], e[N2];
-                pl_nodes<T, N>([&](int l, int j, int i) { return nodes.row[l * N + j][i]; }, bz, gz, u, F);
+                pl_value<T, N>([&](int l, int j, int i) { return nodes.row[l * N + j][i]; }, bz, u);
+                pl_zderivative<T, N>([&](int l, int j, int i) { return nodes.row[l * N + j][i]; }, gz, F);
                 pl_interpolate<T, N>(u, a.t.B);
                 pl_interpolate<T, N>(F, a.t.B);
 #pragma unroll
@@ -311,7 +312,7 @@ namespace mpdg
         for (int qz = 0; qz < N; ++qz)
           {
             T t[N2], tz[N2], cap[N2], k[N2], dk[N2], x[N2] = {}, y[N2];
-            solid_plane<T, N>(a, c, a.t.B + qz * N, a.t.Gz + qz * (N - 1), t, tz, cap);
+            solid_plane<T, N>(a, c, a.t.B + qz * N, a.t.G[2] + qz * (N - 1), t, tz, cap);
 #pragma unroll
             for (int p = 0; p < N2; ++p)
               {

@@ -331,14 +331,11 @@ namespace mpdg
     }
     template <typename T, int N>
     __device__ __forceinline__ void
-    test(T *S, const GaussTab<T, N> &t, T *out)
+    test(T *S, const GaussTab<T, N> &t)
     {
       gp_test<T, N, 2>(S, t.Bt[2]);
       gp_test<T, N, 1>(S, t.Bt[1]);
       gp_test<T, N, 0>(S, t.Bt[0]);
-#pragma unroll
-      for (int q = 0; q < N * N * N; ++q)
-        out[q] = S[q];
     }
     __device__ __forceinline__ double
     point_rsqrt(double x)
@@ -383,22 +380,26 @@ namespace mpdg
       {
         const int       sy = a.g.n[0], sz = a.g.n[0] * a.g.n[1];
         const long long first = K * c.c[0] + (long long)sy * (K * c.c[1]) + (long long)sz * (K * c.c[2]);
+        // values and gradient of u - ref, ref the middle node: interpolated values of nearly equal size cancel
+        const T    ref  = nodes.row[(K / 2) * N + K / 2][K / 2];
+        const auto node = [&](int l, int j, int i) { return nodes.row[l * N + j][i] - ref; };
 #pragma unroll
         for (int q = 0; q < N3; ++q)
           R[q] = T(0);
 #pragma unroll(K == 1 ? 2 : 1)
         for (int qz = 0; qz < N; ++qz)
           {
-            const T *bz = a.t.B + qz * N, *gz = a.t.Gz + qz * (N - 1);
+            const T *bz = a.t.B + qz * N, *gz = a.t.G[2] + qz * (N - 1);
             T        v[3][N2], u[N2], F[N2], S[N2], G[N2];
 #pragma unroll
             for (int d = 0; d < 3; ++d)
               {
                 const double *f = a.n[d] + first;
-                pl_nodes<T, N>([&](int l, int j, int i) { return (T)__ldg(f + (j * sy + l * sz + i)); }, bz, gz, v[d], (T *)nullptr);
+                pl_value<T, N>([&](int l, int j, int i) { return (T)__ldg(f + (j * sy + l * sz + i)); }, bz, v[d]);
                 pl_interpolate<T, N>(v[d], a.t.B);
               }
-            pl_nodes<T, N>([&](int l, int j, int i) { return nodes.row[l * N + j][i]; }, bz, gz, u, F);
+            pl_value<T, N>(node, bz, u);
+            pl_zderivative<T, N>(node, gz, F);
             pl_interpolate<T, N>(u, a.t.B);
             pl_interpolate<T, N>(F, a.t.B);
             // the flux's factor of n_h: c = eps (n_h . grad u) / |n_h|^2, in the right-hand side with the
@@ -410,8 +411,9 @@ namespace mpdg
                 const T nn = fma(v[2][p], v[2][p], fma(v[1][p], v[1][p], v[0][p] * v[0][p]));
                 const T inv = nn > a.tol2 ? point_rsqrt(nn) : a.inv_tol;
                 const T an  = a.eps * (fma(v[2][p], F[p], fma(v[1][p], gy, v[0][p] * gx)) * inv);
-                G[p]        = RHS ? inv * (T(0.5) * (T(1) - u[p] * u[p]) + an) : inv * an;
-                S[p]        = a.mass * u[p];
+                const T w   = u[p] + ref;
+                G[p]        = RHS ? inv * (T(0.5) * (T(1) - w * w) + an) : inv * an;
+                S[p]        = a.mass * w;
                 F[p]        = fma(a.eps_t, F[p], G[p] * v[2][p]);
               }
             pl_divergence<T, N, 0>(S, a.t.P[0], [&](int p) { return fma(a.eps_t, gp_derivative<T, N, 0>(u, a.t.D[0], p), G[p] * v[0][p]); });
@@ -440,15 +442,23 @@ namespace mpdg
         T                        S[N3];
         const unsigned long long bits = band_bits<T, N>(a, c);
         auto in = [&](int q, T x) { return (bits >> q) & 1u ? x : T(0); };
+        // u - ref as in ReinitCellOp
+        const T ref = u[((K / 2) * N + K / 2) * N + K / 2];
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          u[q] -= ref;
         interpolate<T, N>(u, a.t.B);
 #pragma unroll
         for (int q = 0; q < N3; ++q)
-          S[q] = in(q, a.mass * u[q]);
+          S[q] = in(q, a.mass * (u[q] + ref));
         // t.D carries the diffusivity
         gp_divergence<T, N, 0>(S, a.t.P[0], [&](int q) { return in(q, gp_derivative<T, N, 0>(u, a.t.D[0], q)); });
         gp_divergence<T, N, 1>(S, a.t.P[1], [&](int q) { return in(q, gp_derivative<T, N, 1>(u, a.t.D[1], q)); });
         gp_divergence<T, N, 2>(S, a.t.P[2], [&](int q) { return in(q, gp_derivative<T, N, 2>(u, a.t.D[2], q)); });
-        test<T, N>(S, a.t, u);
+        test<T, N>(S, a.t);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          u[q] = S[q];
         return 0.0;
       }
     };
@@ -469,30 +479,46 @@ namespace mpdg
       __device__ __forceinline__ double
       apply(double *u, const PointCell &c) const
       {
-        double             S[N3];
         unsigned long long bits = ~0ull;
         if (a.band_ls)
           bits = band_bits<double, N>(a, c);
-        interpolate<double, N>(u, a.t.B);
+        double inv[NORMALIZED ? N3 : 1];
+        if constexpr (NORMALIZED)
+          {
+            constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
+            double        v[N3];
+#pragma unroll
+            for (int q = 0; q < N3; ++q)
+              v[q] = u[q];
+            gp_gradient<double, N, D1>(v, a.t.B, a.t.G[D1]);
+#pragma unroll
+            for (int q = 0; q < N3; ++q)
+              {
+                inv[q] = v[q] * v[q];
+                v[q]   = u[q];
+              }
+            gp_gradient<double, N, D2>(v, a.t.B, a.t.G[D2]);
+#pragma unroll
+            for (int q = 0; q < N3; ++q)
+              inv[q] = fma(v[q], v[q], inv[q]);
+          }
+        gp_gradient<double, N, DIR>(u, a.t.B, a.t.G[DIR]);
 #pragma unroll
         for (int q = 0; q < N3; ++q)
           {
-            double g = gp_derivative<double, N, DIR>(u, a.t.D[DIR], q);
             if constexpr (NORMALIZED)
               {
-                constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
-                const double  g1 = gp_derivative<double, N, D1>(u, a.t.D[D1], q), g2 = gp_derivative<double, N, D2>(u, a.t.D[D2], q);
-                const double  nn = sqrt(g * g + g1 * g1 + g2 * g2);
-                g *= nn > 1e-16 ? 1.0 / nn : 1e16;
+                const double nn = sqrt(fma(u[q], u[q], inv[q]));
+                u[q] *= nn > 1e-16 ? 1.0 / nn : 1e16;
               }
-            S[q] = (bits >> q) & 1u ? g : 0.0;
+            u[q] = (bits >> q) & 1u ? u[q] : 0.0;
           }
-        test<double, N>(S, a.t, u);
+        test<double, N>(u, a.t);
         return 0.0;
       }
     };
 
-    // -int div(n) phi, n = normalize(n_i, tol) at every DoF; the marching input is n_x.  t.D carries the sign.
+    // -int div(n) phi, n = normalize(n_i, tol) at every DoF; the marching input is n_x.  t.G carries the sign.
     template <int K>
     struct DivergenceCellOp
     {
@@ -525,22 +551,19 @@ namespace mpdg
             v[q] *= inv[q];
             u[q] *= inv[q];
           }
-        interpolate<double, N>(v, a.t.B);
+        gp_gradient<double, N, 2>(v, a.t.B, a.t.G[2]);
+        gp_gradient<double, N, 0>(u, a.t.B, a.t.G[0]);
 #pragma unroll
         for (int q = 0; q < N3; ++q)
-          S[q] = gp_derivative<double, N, 2>(v, a.t.D[2], q);
-        interpolate<double, N>(u, a.t.B);
-#pragma unroll
-        for (int q = 0; q < N3; ++q)
-          S[q] += gp_derivative<double, N, 0>(u, a.t.D[0], q);
+          S[q] = v[q] + u[q];
         field_nodes<double, N>(a.n[1], a.g, c, v);
 #pragma unroll
         for (int q = 0; q < N3; ++q)
           v[q] *= inv[q];
-        interpolate<double, N>(v, a.t.B);
+        gp_gradient<double, N, 1>(v, a.t.B, a.t.G[1]);
 #pragma unroll
         for (int q = 0; q < N3; ++q)
-          S[q] += gp_derivative<double, N, 1>(v, a.t.D[1], q);
+          S[q] += v[q];
         if (a.band_ls)
           {
             const unsigned long long bits = band_bits<double, N>(a, c);
@@ -548,7 +571,10 @@ namespace mpdg
             for (int q = 0; q < N3; ++q)
               S[q] = (bits >> q) & 1u ? S[q] : 0.0;
           }
-        test<double, N>(S, a.t, u);
+        test<double, N>(S, a.t);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
+          u[q] = S[q];
         return 0.0;
       }
     };
@@ -604,7 +630,7 @@ namespace mpdg
       a.t.fill(t, h.hlen);
       if (h.normal[0] == nullptr) // the banded form's flux: D carries the diffusivity
         for (int d = 0; d < 3; ++d)
-          gp_on_differences<T, N>(t.Dq, h.scale * h.eps_tangential / h.hlen[d], a.t.D[d]);
+          gp_on_differences<T, N>(t.ext.Dq, (long double)h.scale * h.eps_tangential / h.hlen[d], a.t.D[d]);
       a.eps_t    = (T)((mode == 1 ? -1.0 : h.scale) * h.eps_tangential);
       a.eps      = (T)((mode == 1 ? -1.0 : h.scale) * (h.eps_normal - h.eps_tangential));
       a.mass     = mode == 1 ? T(0) : (T)(h.scale / h.dt);
@@ -757,7 +783,7 @@ namespace mpdg
         {
           a.n[d] = in[d];
           for (int i = 0; i < N * (N - 1); ++i)
-            a.t.D[d][i] = -a.t.D[d][i];
+            a.t.G[d][i] = -a.t.G[d][i];
         }
       a.tol2    = tol * tol;
       a.inv_tol = 1.0 / tol;

@@ -11,10 +11,11 @@ namespace mpdg
 {
   namespace
   {
+    template <typename real>
     void
-    legendre(int n, double x, double &p, double &dp)
+    legendre(int n, real x, real &p, real &dp)
     {
-      double p0 = 1.0, p1 = x;
+      real p0 = 1.0, p1 = x;
       if (n == 0)
         {
           p  = 1.0;
@@ -23,7 +24,7 @@ namespace mpdg
         }
       for (int k = 2; k <= n; ++k)
         {
-          const double p2 = ((2.0 * k - 1.0) * x * p1 - (k - 1.0) * p0) / k;
+          const real p2 = ((2.0 * k - 1.0) * x * p1 - (k - 1.0) * p0) / k;
           p0              = p1;
           p1              = p2;
         }
@@ -32,22 +33,23 @@ namespace mpdg
     }
 
     // interior Gauss-Lobatto points: roots of P_k' by Newton, with P_k'' from Legendre's equation
+    template <typename real>
     void
-    lobatto(int k, double *x01)
+    lobatto(int k, real *x01)
     {
       x01[0] = 0.0;
       x01[k] = 1.0;
       for (int i = 1; i < k; ++i)
         {
-          double x = -std::cos(M_PI * i / k);
+          real x = -std::cos(real(M_PI) * i / k);
           for (int it = 0; it < 200; ++it)
             {
-              double p, dp;
+              real p, dp;
               legendre(k, x, p, dp);
-              const double ddp = (2.0 * x * dp - k * (k + 1.0) * p) / (1.0 - x * x);
-              const double dx  = dp / ddp;
+              const real ddp = (2.0 * x * dp - k * (k + 1.0) * p) / (1.0 - x * x);
+              const real dx  = dp / ddp;
               x -= dx;
-              if (std::abs(dx) < 1e-17)
+              if (std::abs(dx) < real(1e-17))
                 break;
             }
           x01[i] = 0.5 * (x + 1.0);
@@ -55,19 +57,20 @@ namespace mpdg
       std::sort(x01, x01 + k + 1);
     }
 
+    template <typename real>
     void
-    gauss(int n, double *x01, double *w01)
+    gauss(int n, real *x01, real *w01)
     {
       for (int i = 0; i < n; ++i)
         {
-          double x = -std::cos(M_PI * (i + 0.75) / (n + 0.5));
-          double p = 0.0, dp = 1.0;
+          real x = -std::cos(real(M_PI) * (i + 0.75) / (n + 0.5));
+          real p = 0.0, dp = 1.0;
           for (int it = 0; it < 200; ++it)
             {
               legendre(n, x, p, dp);
-              const double dx = p / dp;
+              const real dx = p / dp;
               x -= dx;
-              if (std::abs(dx) < 1e-17)
+              if (std::abs(dx) < real(1e-17))
                 break;
             }
           legendre(n, x, p, dp);
@@ -83,8 +86,9 @@ namespace mpdg
             }
     }
 
+    template <typename real>
     void
-    lagrange(int n, const double *x, int i, double t, double &val, double &der)
+    lagrange(int n, const real *x, int i, real t, real &val, real &der)
     {
       val = 1.0;
       for (int j = 0; j < n; ++j)
@@ -95,7 +99,7 @@ namespace mpdg
         {
           if (m == i)
             continue;
-          double prod = 1.0 / (x[i] - x[m]);
+          real prod = 1.0 / (x[i] - x[m]);
           for (int j = 0; j < n; ++j)
             if (j != i && j != m)
               prod *= (t - x[j]) / (x[i] - x[j]);
@@ -240,6 +244,22 @@ namespace mpdg
         }
     }
 
+    template <typename real>
+    void
+    points(int degree, real *nodes, real *qp, real *qw, real *B, real *G, real *Dq)
+    {
+      const int n = degree + 1;
+      lobatto(degree, nodes);
+      gauss(n, qp, qw);
+      for (int q = 0; q < n; ++q)
+        for (int i = 0; i < n; ++i)
+          {
+            real v;
+            lagrange(n, nodes, i, qp[q], B[q * n + i], G[q * n + i]);
+            lagrange(n, qp, i, qp[q], v, Dq[q * n + i]);
+          }
+    }
+
     Tables1D
     build(int degree)
     {
@@ -248,18 +268,9 @@ namespace mpdg
       t.n         = n;
       t.ne        = (n + 1) / 2;
       t.no        = n / 2;
-      lobatto(degree, t.nodes);
-      gauss(n, t.qp, t.qw);
-      for (int q = 0; q < n; ++q)
-        for (int i = 0; i < n; ++i)
-          lagrange(n, t.nodes, i, t.qp[q], t.B[q * n + i], t.G[q * n + i]);
-      for (int q = 0; q < n; ++q)
-        for (int r = 0; r < n; ++r)
-          {
-            double v, d;
-            lagrange(n, t.qp, r, t.qp[q], v, d);
-            t.Dq[q * n + r] = d;
-          }
+      points<double>(degree, t.nodes, t.qp, t.qw, t.B, t.G, t.Dq);
+      long double nodes[MAX_N], qp[MAX_N];
+      points<long double>(degree, nodes, qp, t.ext.qw, t.ext.B, t.ext.G, t.ext.Dq);
       for (int i = 0; i < n; ++i)
         for (int j = 0; j < n; ++j)
           {

@@ -26,6 +26,11 @@ namespace mpdg
     double WE[MAX_N * MAX_N]{};
     double WO[MAX_N * MAX_N]{};
     double lam[MAX_N]{}; // eigenvalues in modal order: even modes first, then odd
+    // weights, B, G and Dq in extended precision, for tables of products that are rounded once
+    struct
+    {
+      long double qw[MAX_N]{}, B[MAX_N * MAX_N]{}, G[MAX_N * MAX_N]{}, Dq[MAX_N * MAX_N]{};
+    } ext;
   };
 
   // Builds and caches the tables of one degree (thread-safe after the first call per degree).
