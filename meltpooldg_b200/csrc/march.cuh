@@ -323,11 +323,39 @@ namespace mpdg
     const T *row[(K + 1) * (K + 1)];
   };
 
+  // Results of a cell operator: 1, or Op::OUT of them
+  template <class Op, class = void>
+  struct MarchOutputs
+  {
+    static constexpr int value = 1;
+    struct State
+    {};
+  };
+  template <class Op>
+  struct MarchOutputs<Op, std::void_t<decltype(Op::OUT)>>
+  {
+    static constexpr int value = Op::OUT;
+    using State                = typename Op::State;
+  };
+  template <int M, int OUT, class Op, typename T, class Nodes, class State, class Finish>
+  __device__ __forceinline__ void
+  march_components(const Op &op, T *u, const Nodes &nodes, State &state, const Finish &finish)
+  {
+    if constexpr (M < OUT)
+      {
+        op.template component<M>(u, nodes, state);
+        finish(M, op.out(M));
+        march_components<M + 1, OUT>(op, u, nodes, state, finish);
+      }
+  }
+
   // The marching body.  Cell operator: op.apply<DOT>(u, op.load(valid, cx, cy, cz)) in place on (K+1)^3 values.
   // With DOT the cell operator returns the cell's form src_c^T A src_c and the sum over the segment goes
   // to the fused dot product (release_ticket_dot).
   // An operator with Op::NODES instead has op.apply(u, nodes, op.load(...)): it reads its input through
   // MarchNodes and only writes u.
+  // An operator with Op::OUT results (NODES) has op.prepare(nodes, pre, state), op.component<m>(u, nodes, state)
+  // and the output vectors op.out(m) instead: result after result of a layer is exchanged and written.
   // MASKABLE: the operator may carry per-DoF constraint flags (GridDesc::cmask) besides the faces.
   template <int K, typename T, OutMode MODE, class Op, bool DOT = false, bool MASKABLE = false>
   __device__ __forceinline__ void
@@ -384,10 +412,13 @@ namespace mpdg
     // Dirichlet planes through the cell
     const bool cI0 = br.con_lo[0] && cx == 0, cIK = br.con_hi[0] && cx == g.m[0] - 1;
     const bool cJ0 = br.con_lo[1] && cy == 0, cJK = br.con_hi[1] && cy == g.m[1] - 1;
-    T carry[K * K];
+    constexpr int OUT = MarchOutputs<Op>::value;
+    T             carry[OUT][K * K];
 #pragma unroll
-    for (int q = 0; q < K * K; ++q)
-      carry[q] = T(0);
+    for (int m = 0; m < OUT; ++m)
+#pragma unroll
+      for (int q = 0; q < K * K; ++q)
+        carry[m][q] = T(0);
     const int wbase  = br.index(0, K * warp, 0); // first point of the warp's cell row
     int       slot0  = 0;                          // ring slot of the layer's low plane
     for (int lz = 0; lz < nlayers; ++lz)
@@ -402,6 +433,7 @@ namespace mpdg
         const bool cL0 = br.con_lo[2] && cz == 0, cLK = br.con_hi[2] && cz == g.m[2] - 1;
         T                u[N * N * N];
         MarchNodes<K, T> nodes;
+        typename MarchOutputs<Op>::State state;
 #pragma unroll
         for (int l = 0; l < N; ++l)
           {
@@ -417,6 +449,144 @@ namespace mpdg
         slot0 += K;
         if (slot0 >= NRING)
           slot0 -= NRING;
+        // exchange of result m (u) with the neighbouring cells and write-out to out
+        auto finish = [&](const int m, T *out) {
+          // x: lane t adds lane t-1's x = K face
+#pragma unroll
+          for (int q = 0; q < N * N; ++q)
+            {
+              const T v = __shfl_up_sync(0xffffffffu, u[q * N + K], 1);
+              if (lane > 0)
+                u[q * N] += v;
+            }
+          // y: warp w hands its y = K face to warp w + 1 (the last warp adds its own to dst below)
+          T *yx = yx0 + ((OUT * lz + m) & 1) * LAY::YX;
+#pragma unroll
+          for (int l = 0; l < N; ++l)
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+              yx[((warp * N + l) * K + i) * 32 + lane] = u[(l * N + K) * N + i];
+          if constexpr (MODE != OutMode::Add)
+            if (lz == 0 && m == 0 && br.has_lower_neighbour())
+              column_wait_lower<K>(br, g, s);
+          __syncthreads();
+          // every thread has read the layer's planes: those that the layer after next needs not are free
+          if (m == OUT - 1 && warp == 0 && lz + 2 < nlayers)
+            march_stage<K, T>(br, src, n_src, base, K * (lz + 2) + 1, K * (lz + 3) + 1, ring, &bars[lz & 1]);
+          if (warp > 0)
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+#pragma unroll
+              for (int i = 0; i < K; ++i)
+                u[(l * N) * N + i] += yx[(((warp - 1) * N + l) * K + i) * 32 + lane];
+          // z: add the carried face, carry this layer's z = K face
+#pragma unroll
+          for (int j = 0; j < K; ++j)
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+              {
+                u[j * N + i] += carry[m][j * K + i];
+                carry[m][j * K + i] = u[(K * N + j) * N + i];
+              }
+          // ---- write-out.  Every face point of the segment was initialised by its owner
+          // (column_init_publish), so a face point is an atomic add (skipped on constrained rows) and an
+          // interior point a plain store; interior points are never constrained (Dirichlet planes are
+          // domain faces).
+          auto write_out = [&](auto flagged) {
+              constexpr bool CM    = decltype(flagged)::value;
+              const int      cbase = wbase + K * lane + br.sz * (K * lz);
+              T             *d0    = out + cbase;
+              const bool     x_low = lane == 0;
+              auto store = [&](int i, int j, int l) {
+                const int off = j * br.sy + l * br.sz + i;
+                const T   v   = u[(l * N + j) * N + i];
+                bool con = false;
+                if constexpr (CM)
+                  con = g.cmask[cbase + off] != 0;
+                if constexpr (MODE == OutMode::Set)
+                  d0[off] = con ? T(0) : v;
+                else if constexpr (MODE == OutMode::Add)
+                  {
+                    // a reduction without a return value: nothing waits for the old value
+                    if (!con)
+                      atomicAdd(d0 + off, v);
+                  }
+                else
+                  d0[off] = con ? bvec[cbase + off] : bvec[cbase + off] + v;
+              };
+              auto add = [&](int i, int j, int l) {
+                const int off = j * br.sy + l * br.sz + i;
+                if constexpr (CM)
+                  if (g.cmask[cbase + off])
+                    return;
+                atomicAdd(d0 + off, u[(l * N + j) * N + i]);
+              };
+#pragma unroll
+              for (int l = 0; l < K; ++l)
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+                  {
+                    if ((j == 0 && warp == 0) || (l == 0 && lz == 0))
+                      {
+                        if (!((j == 0 && cJ0) || (l == 0 && cL0)))
+#pragma unroll
+                          for (int i = 0; i < K; ++i)
+                            if (!(i == 0 && cI0))
+                              add(i, j, l);
+                      }
+                    else
+                      {
+                        if (!x_low)
+                          store(0, j, l);
+#pragma unroll
+                        for (int i = 1; i < K; ++i)
+                          store(i, j, l);
+                      }
+                  }
+              if (x_low && !cI0)
+#pragma unroll
+                for (int l = 0; l < K; ++l)
+#pragma unroll
+                  for (int j = 0; j < K; ++j)
+                    if (!((j == 0 && warp == 0) || (l == 0 && lz == 0)))
+                      add(0, j, l);
+              if (last_lane && !cIK)
+#pragma unroll
+                for (int l = 0; l < N; ++l)
+#pragma unroll
+                  for (int j = 0; j < N; ++j)
+                    if (!((j == 0 && cJ0) || (j == K && cJK) || (l == 0 && cL0) || (l == K && cLK)))
+                      add(K, j, l);
+              if (last_warp && !cJK)
+#pragma unroll
+                for (int l = 0; l < N; ++l)
+                  if (!((l == 0 && cL0) || (l == K && cLK)))
+#pragma unroll
+                    for (int i = 0; i < K; ++i)
+                      if (!(i == 0 && cI0))
+                        add(i, K, l);
+              if (last_layer && !cLK)
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+                  if (!(j == 0 && cJ0))
+#pragma unroll
+                    for (int i = 0; i < K; ++i)
+                      if (!(i == 0 && cI0))
+                        add(i, j, K);
+          };
+          if (vxy)
+            {
+              if constexpr (MASKABLE)
+                {
+                  if (g.cmask != nullptr)
+                    write_out(std::true_type());
+                  else
+                    write_out(std::false_type());
+                }
+              else
+                write_out(std::false_type());
+            }
+        };
         if constexpr (Op::NODES)
           {
             // constrained entry (i, j, l) of the cell: Dirichlet planes, per-DoF flags
@@ -442,7 +612,10 @@ namespace mpdg
                           const_cast<T *>(nodes.row[l * N + j])[i] = T(0);
                 __syncthreads();
               }
-            op.apply(u, nodes, pre);
+            if constexpr (OUT == 1)
+              op.apply(u, nodes, pre);
+            else
+              op.prepare(nodes, pre, state);
           }
         else
           {
@@ -483,141 +656,10 @@ namespace mpdg
             else
               op.template apply<false>(u, pre);
           }
-        // x: lane t adds lane t-1's x = K face
-#pragma unroll
-        for (int q = 0; q < N * N; ++q)
-          {
-            const T v = __shfl_up_sync(0xffffffffu, u[q * N + K], 1);
-            if (lane > 0)
-              u[q * N] += v;
-          }
-        // y: warp w hands its y = K face to warp w + 1 (the last warp adds its own to dst below)
-        T *yx = yx0 + (lz & 1) * LAY::YX;
-#pragma unroll
-        for (int l = 0; l < N; ++l)
-#pragma unroll
-          for (int i = 0; i < K; ++i)
-            yx[((warp * N + l) * K + i) * 32 + lane] = u[(l * N + K) * N + i];
-        if constexpr (MODE != OutMode::Add)
-          if (lz == 0 && br.has_lower_neighbour())
-            column_wait_lower<K>(br, g, s);
-        __syncthreads();
-        // every thread has read the layer's planes: those that the layer after next needs not are free
-        if (warp == 0 && lz + 2 < nlayers)
-          march_stage<K, T>(br, src, n_src, base, K * (lz + 2) + 1, K * (lz + 3) + 1, ring, &bars[lz & 1]);
-        if (warp > 0)
-#pragma unroll
-          for (int l = 0; l < N; ++l)
-#pragma unroll
-            for (int i = 0; i < K; ++i)
-              u[(l * N) * N + i] += yx[(((warp - 1) * N + l) * K + i) * 32 + lane];
-        // z: add the carried face, carry this layer's z = K face
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-          for (int i = 0; i < K; ++i)
-            {
-              u[j * N + i] += carry[j * K + i];
-              carry[j * K + i] = u[(K * N + j) * N + i];
-            }
-        // ---- write-out.  Every face point of the segment was initialised by its owner
-        // (column_init_publish), so a face point is an atomic add (skipped on constrained rows) and an
-        // interior point a plain store; interior points are never constrained (Dirichlet planes are
-        // domain faces).
-        auto write_out = [&](auto flagged) {
-            constexpr bool CM    = decltype(flagged)::value;
-            const int      cbase = wbase + K * lane + br.sz * (K * lz);
-            T             *d0    = dst + cbase;
-            const bool     x_low = lane == 0;
-            auto store = [&](int i, int j, int l) {
-              const int off = j * br.sy + l * br.sz + i;
-              const T   v   = u[(l * N + j) * N + i];
-              bool con = false;
-              if constexpr (CM)
-                con = g.cmask[cbase + off] != 0;
-              if constexpr (MODE == OutMode::Set)
-                d0[off] = con ? T(0) : v;
-              else if constexpr (MODE == OutMode::Add)
-                {
-                  // a reduction without a return value: nothing waits for the old value
-                  if (!con)
-                    atomicAdd(d0 + off, v);
-                }
-              else
-                d0[off] = con ? bvec[cbase + off] : bvec[cbase + off] + v;
-            };
-            auto add = [&](int i, int j, int l) {
-              const int off = j * br.sy + l * br.sz + i;
-              if constexpr (CM)
-                if (g.cmask[cbase + off])
-                  return;
-              atomicAdd(d0 + off, u[(l * N + j) * N + i]);
-            };
-#pragma unroll
-            for (int l = 0; l < K; ++l)
-#pragma unroll
-              for (int j = 0; j < K; ++j)
-                {
-                  if ((j == 0 && warp == 0) || (l == 0 && lz == 0))
-                    {
-                      if (!((j == 0 && cJ0) || (l == 0 && cL0)))
-#pragma unroll
-                        for (int i = 0; i < K; ++i)
-                          if (!(i == 0 && cI0))
-                            add(i, j, l);
-                    }
-                  else
-                    {
-                      if (!x_low)
-                        store(0, j, l);
-#pragma unroll
-                      for (int i = 1; i < K; ++i)
-                        store(i, j, l);
-                    }
-                }
-            if (x_low && !cI0)
-#pragma unroll
-              for (int l = 0; l < K; ++l)
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-                  if (!((j == 0 && warp == 0) || (l == 0 && lz == 0)))
-                    add(0, j, l);
-            if (last_lane && !cIK)
-#pragma unroll
-              for (int l = 0; l < N; ++l)
-#pragma unroll
-                for (int j = 0; j < N; ++j)
-                  if (!((j == 0 && cJ0) || (j == K && cJK) || (l == 0 && cL0) || (l == K && cLK)))
-                    add(K, j, l);
-            if (last_warp && !cJK)
-#pragma unroll
-              for (int l = 0; l < N; ++l)
-                if (!((l == 0 && cL0) || (l == K && cLK)))
-#pragma unroll
-                  for (int i = 0; i < K; ++i)
-                    if (!(i == 0 && cI0))
-                      add(i, K, l);
-            if (last_layer && !cLK)
-#pragma unroll
-              for (int j = 0; j < K; ++j)
-                if (!(j == 0 && cJ0))
-#pragma unroll
-                  for (int i = 0; i < K; ++i)
-                    if (!(i == 0 && cI0))
-                      add(i, j, K);
-        };
-        if (vxy)
-          {
-            if constexpr (MASKABLE)
-              {
-                if (g.cmask != nullptr)
-                  write_out(std::true_type());
-                else
-                  write_out(std::false_type());
-              }
-            else
-              write_out(std::false_type());
-          }
+        if constexpr (OUT == 1)
+          finish(0, dst);
+        else
+          march_components<0, OUT>(op, u, nodes, state, finish);
       }
     if constexpr (DOT)
       release_ticket_dot<MARCH_NT>(s, dot, br.id, dsum, s_red, s_ticket);

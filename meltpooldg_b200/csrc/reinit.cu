@@ -368,8 +368,9 @@ namespace mpdg
     struct ReinitCellOp
     {
       static constexpr int  N = K + 1, N2 = N * N, N3 = N * N * N;
-      static constexpr bool HEAVY = true, NODES = true;
-      const PointArgs<T, N> &a;
+      static constexpr bool HEAVY = true, NODES = true, SPLIT = false;
+      using Args = PointArgs<T, N>;
+      const Args &a;
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
@@ -427,9 +428,10 @@ namespace mpdg
     template <int K, typename T>
     struct BandCellOp
     {
-      static constexpr bool HEAVY = false, NODES = false;
+      static constexpr bool HEAVY = false, NODES = false, SPLIT = false;
       static constexpr int N = K + 1, N3 = N * N * N;
-      const PointArgs<T, N> &a;
+      using Args = PointArgs<T, N>;
+      const Args &a;
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
@@ -463,58 +465,107 @@ namespace mpdg
       }
     };
 
-    // int (grad psi)_DIR phi, in the band if there is one; NORMALIZED: the unit gradient (|.| > 1e-16)
-    template <int K, int DIR, bool NORMALIZED>
+    // int grad psi phi, in the band if there is one, to three vectors; NORMALIZED: the unit gradient
+    // (|.| > 1e-16).  One launch, the components finished one after the other, or (SPLIT: unit gradient at
+    // k = 3, whose 192 values do not fit the registers) by CTAs of their own.  FE_Q(1) 33x66x80: gradient 33 us as three launches, 19 as one; unit gradient,
+    // which each of the three formed anew, 62 and 30; FE_Q(2) 80x64x48: 66 and 52, 225 and 125.
+    template <int K>
+    struct GradientArgs : PointArgs<double, K + 1>
+    {
+      double *out[3];
+    };
+    template <int K, bool NORMALIZED>
     struct GradientCellOp
     {
-      static constexpr bool HEAVY = false, NODES = false;
-      static constexpr int N = K + 1, N3 = N * N * N;
-      const PointArgs<double, N> &a;
+      static constexpr bool HEAVY = NORMALIZED, NODES = true, SPLIT = NORMALIZED && K == 3;
+      static constexpr int  N = K + 1, N3 = N * N * N, OUT = SPLIT ? 1 : 3;
+      using Args = GradientArgs<K>;
+      struct State
+      {
+        unsigned long long bits;
+        double             g[NORMALIZED && !SPLIT ? 3 : 1][NORMALIZED && !SPLIT ? N3 : 1]; // the unit gradient
+      };
+      const Args &a;
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
         return point_cell<double, N>(a.g, cx, cy, cz);
       }
-      template <bool DOT>
-      __device__ __forceinline__ double
-      apply(double *u, const PointCell &c) const
+      __device__ __forceinline__ double *
+      out(int m) const
       {
-        unsigned long long bits = ~0ull;
-        if (a.band_ls)
-          bits = band_bits<double, N>(a, c);
-        double inv[NORMALIZED ? N3 : 1];
-        if constexpr (NORMALIZED)
+        return a.out[m];
+      }
+      // put(q, gx, gy, gz): the unit gradient at the points, from u - ref as in ReinitCellOp
+      template <class Put>
+      __device__ __forceinline__ void
+      unit_gradient(const MarchNodes<K, double> &nodes, const Put &put) const
+      {
+        const double ref = nodes.row[(K / 2) * N + K / 2][K / 2];
+        double       v[N3];
+#pragma unroll
+        for (int r = 0; r < N * N; ++r)
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            v[r * N + i] = nodes.row[r][i] - ref;
+        interpolate<double, N>(v, a.t.B);
+#pragma unroll
+        for (int q = 0; q < N3; ++q)
           {
-            constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
-            double        v[N3];
-#pragma unroll
-            for (int q = 0; q < N3; ++q)
-              v[q] = u[q];
-            gp_gradient<double, N, D1>(v, a.t.B, a.t.G[D1]);
-#pragma unroll
-            for (int q = 0; q < N3; ++q)
-              {
-                inv[q] = v[q] * v[q];
-                v[q]   = u[q];
-              }
-            gp_gradient<double, N, D2>(v, a.t.B, a.t.G[D2]);
-#pragma unroll
-            for (int q = 0; q < N3; ++q)
-              inv[q] = fma(v[q], v[q], inv[q]);
+            const double gx = gp_derivative<double, N, 0>(v, a.t.D[0], q), gy = gp_derivative<double, N, 1>(v, a.t.D[1], q),
+                         gz = gp_derivative<double, N, 2>(v, a.t.D[2], q);
+            const double nn = sqrt(fma(gz, gz, fma(gy, gy, gx * gx))), f = nn > 1e-16 ? 1.0 / nn : 1e16;
+            put(q, f * gx, f * gy, f * gz);
           }
-        gp_gradient<double, N, DIR>(u, a.t.B, a.t.G[DIR]);
+      }
+      __device__ __forceinline__ unsigned long long
+      band(const PointCell &c) const
+      {
+        return a.band_ls ? band_bits<double, N>(a, c) : ~0ull;
+      }
+      __device__ __forceinline__ void
+      prepare(const MarchNodes<K, double> &nodes, const PointCell &c, State &s) const
+      {
+        s.bits = band(c);
+        if constexpr (NORMALIZED)
+          unit_gradient(nodes, [&](int q, double gx, double gy, double gz) {
+            s.g[0][q] = gx;
+            s.g[1][q] = gy;
+            s.g[2][q] = gz;
+          });
+      }
+      template <int DIR>
+      __device__ __forceinline__ void
+      component(double *u, const MarchNodes<K, double> &nodes, State &s) const
+      {
+        if constexpr (!NORMALIZED)
+          {
+#pragma unroll
+            for (int r = 0; r < N * N; ++r)
+#pragma unroll
+              for (int i = 0; i < N; ++i)
+                u[r * N + i] = nodes.row[r][i];
+            gp_gradient<double, N, DIR>(u, a.t.B, a.t.G[DIR]);
+          }
 #pragma unroll
         for (int q = 0; q < N3; ++q)
           {
             if constexpr (NORMALIZED)
-              {
-                const double nn = sqrt(fma(u[q], u[q], inv[q]));
-                u[q] *= nn > 1e-16 ? 1.0 / nn : 1e16;
-              }
-            u[q] = (bits >> q) & 1u ? u[q] : 0.0;
+              u[q] = s.g[DIR][q];
+            u[q] = (s.bits >> q) & 1u ? u[q] : 0.0;
           }
         test<double, N>(u, a.t);
-        return 0.0;
+      }
+      // SPLIT: the component of the CTA
+      __device__ __forceinline__ void
+      apply(double *u, const MarchNodes<K, double> &nodes, const PointCell &c) const
+      {
+        const unsigned long long bits = band(c);
+        const unsigned           dir  = blockIdx.y;
+        unit_gradient(nodes, [&](int q, double gx, double gy, double gz) {
+          u[q] = (bits >> q) & 1u ? (dir == 0 ? gx : dir == 1 ? gy : gz) : 0.0;
+        });
+        test<double, N>(u, a.t);
       }
     };
 
@@ -522,9 +573,10 @@ namespace mpdg
     template <int K>
     struct DivergenceCellOp
     {
-      static constexpr bool HEAVY = false, NODES = false;
+      static constexpr bool HEAVY = false, NODES = false, SPLIT = false;
       static constexpr int N = K + 1, N3 = N * N * N;
-      const PointArgs<double, N> &a;
+      using Args = PointArgs<double, N>;
+      const Args &a;
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
@@ -592,19 +644,22 @@ namespace mpdg
 
     template <int K, typename T, OutMode MODE, class Op>
     __global__ void __launch_bounds__(MARCH_NT, PointMinBlocks<K, T, Op::HEAVY>::value)
-    reinit_march_kernel(const __grid_constant__ PointArgs<T, K + 1> a)
+    reinit_march_kernel(const __grid_constant__ typename Op::Args a)
     {
       extern __shared__ __align__(16) unsigned char smem_raw[];
       __shared__ unsigned                        s_ticket;
       __shared__ __align__(8) unsigned long long s_bars[2];
       Op                                         op{a};
-      march_body<K, T, MODE, Op, false, true>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
+      T                                         *dst = a.dst;
+      if constexpr (Op::SPLIT)
+        dst = a.out[blockIdx.y];
+      march_body<K, T, MODE, Op, false, true>(a.g, a.s, a.src, dst, a.b, a.mask_src != 0, op,
                                               reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
     }
 
     template <int K, typename T, OutMode MODE, class Op>
     cudaError_t
-    launch_point_kernel(PointArgs<T, K + 1> &a, cudaStream_t s)
+    launch_point_kernel(typename Op::Args &a, cudaStream_t s)
     {
       auto                                   kern = reinit_march_kernel<K, T, MODE, Op>;
       static std::atomic<unsigned long long> devices{0};
@@ -612,7 +667,7 @@ namespace mpdg
       if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
         return e;
       const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, PointMinBlocks<K, T, Op::HEAVY>::value);
-      kern<<<ctas, MARCH_NT, bytes, s>>>(a);
+      kern<<<dim3(ctas, Op::SPLIT ? 3 : 1), MARCH_NT, bytes, s>>>(a);
       return cudaGetLastError();
     }
 
@@ -747,21 +802,6 @@ namespace mpdg
 
   namespace
   {
-    template <int K, bool NORMALIZED>
-    cudaError_t
-    launch_normal_rhs(PointArgs<double, K + 1> &a, double *const out[3], cudaStream_t s)
-    {
-      cudaError_t e;
-      a.dst = out[0];
-      if ((e = launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 0, NORMALIZED>>(a, s)) != cudaSuccess)
-        return e;
-      a.dst = out[1];
-      if ((e = launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 1, NORMALIZED>>(a, s)) != cudaSuccess)
-        return e;
-      a.dst = out[2];
-      return launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, 2, NORMALIZED>>(a, s);
-    }
-
     template <int K>
     cudaError_t
     launch_level_set_rhs(const GridDesc &g, const SyncDesc &sync, const double hlen[3], int mode, int normalized, double tol,
@@ -769,7 +809,7 @@ namespace mpdg
                          double band)
     {
       constexpr int        N = K + 1;
-      PointArgs<double, N> a{};
+      GradientArgs<K> a{};
       a.g = g;
       a.s = sync;
       a.t.fill(tables(K), hlen);
@@ -778,7 +818,12 @@ namespace mpdg
       a.band_ls  = band > 0.0 ? band_ls : nullptr;
       a.band     = band;
       if (mode == 0)
-        return normalized ? launch_normal_rhs<K, true>(a, out, s) : launch_normal_rhs<K, false>(a, out, s);
+        {
+          for (int d = 0; d < 3; ++d)
+            a.out[d] = out[d];
+          return normalized ? launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, true>>(a, s) :
+                              launch_point_kernel<K, double, OutMode::Add, GradientCellOp<K, false>>(a, s);
+        }
       for (int d = 0; d < 3; ++d)
         {
           a.n[d] = in[d];
@@ -794,7 +839,7 @@ namespace mpdg
 
   // Right-hand sides of the normal-vector and curvature projections:
   //   mode 0: dst_d += int g_d phi, g = grad psi, or normalize(grad psi, 1e-16) when normalized
-  //           (normal_vector_operator.cpp:160-240), one launch per component
+  //           (normal_vector_operator.cpp:160-240)
   //   mode 1: dst   = -int div(n) phi with n = normalize(n_i, tol) at every DoF
   //           (curvature_operator.cpp:190-255)
   // Narrow band (normal_vector_operator.cpp:184-191, curvature_operator.cpp:209-214): the gradient or the
