@@ -49,6 +49,75 @@ namespace mpdg
       T             Vend[2 * N], Dend[2 * N]; // basis values / derivatives at x = 0 and x = 1
     };
 
+    // cell of a lane (a lane outside the mesh reads the fields of the nearest cell), and the values of a
+    // plainly read field at the cell's nodes or Gauss points
+    struct PointCell
+    {
+      int c[3];
+    };
+    template <typename T, int N>
+    __device__ __forceinline__ PointCell
+    point_cell(const GridDesc &g, int cx, int cy, int cz)
+    {
+      return PointCell{{min(cx, g.m[0] - 1), min(cy, g.m[1] - 1), cz}};
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    field_nodes(const double *f, const GridDesc &g, const PointCell &c, T *v)
+    {
+      constexpr int K  = N - 1;
+      const int     sy = g.n[0], sz = g.n[0] * g.n[1];
+      f += K * c.c[0] + (long long)sy * (K * c.c[1]) + (long long)sz * (K * c.c[2]);
+#pragma unroll
+      for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+            v[(l * N + j) * N + i] = (T)__ldg(f + (j * sy + l * sz + i));
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    interpolate(T *v, const T *B)
+    {
+      gp_interpolate<T, N, 0>(v, B);
+      gp_interpolate<T, N, 1>(v, B);
+      gp_interpolate<T, N, 2>(v, B);
+    }
+    template <typename T, int N>
+    __device__ __forceinline__ void
+    test(T *S, const GaussTab<T, N> &t)
+    {
+      gp_test<T, N, 2>(S, t.Bt[2]);
+      gp_test<T, N, 1>(S, t.Bt[1]);
+      gp_test<T, N, 0>(S, t.Bt[0]);
+    }
+    __device__ __forceinline__ double
+    point_rsqrt(double x)
+    {
+      return rsqrt(x);
+    }
+    __device__ __forceinline__ float
+    point_rsqrt(float x)
+    {
+      return 1.0f / sqrtf(x);
+    }
+    // Points of the narrow band, one bit per Gauss point.  The apply, the right-hand sides and the diagonal all ask
+    // here: a point within rounding of the threshold has to be in all of them or in none.
+    template <typename T, int N>
+    __device__ __forceinline__ unsigned long long
+    band_bits(const double *ls, T band, const T *B, const GridDesc &g, const PointCell &c)
+    {
+      T v[N * N * N];
+      field_nodes<T, N>(ls, g, c, v);
+      interpolate<T, N>(v, B);
+      unsigned long long bits = 0;
+#pragma unroll
+      for (int q = 0; q < N * N * N; ++q)
+        bits |= (unsigned long long)(fabs(v[q]) < band ? 1u : 0u) << q;
+      return bits;
+    }
+
     // Diagonal of the tangent (and of the banded isotropic form), one thread per cell, point by point
     template <int K, typename T>
     __global__ void __launch_bounds__(128)
@@ -62,7 +131,7 @@ namespace mpdg
           const int cx = (int)(c % m0), cy = (int)((c / m0) % m1), cz = (int)(c / ((long long)m0 * m1));
           long long idx[N3];
           bool      con[N3];
-          T         R[N3], ls[N3];
+          T         R[N3];
 #pragma unroll
           for (int l = 0; l < N; ++l)
 #pragma unroll
@@ -76,14 +145,15 @@ namespace mpdg
                   idx[q]             = id;
                   con[q]             = is_constrained(a.g, I, J, L, id);
                   R[q]               = T(0);
-                  ls[q]              = a.band_ls ? (T)a.band_ls[id] : T(0); // read plainly
                 }
+          const unsigned long long bits =
+            a.band_ls ? band_bits<T, N>(a.band_ls, a.band, a.B, a.g, PointCell{{cx, cy, cz}}) : ~0ull;
           for (int qz = 0; qz < N; ++qz)
             for (int qy = 0; qy < N; ++qy)
               for (int qx = 0; qx < N; ++qx)
                 {
-                  // the normal field (none in the isotropic form) and the level set at the Gauss point
-                  T          nv[3] = {T(0), T(0), T(0)}, lq = T(0);
+                  // the normal field (none in the isotropic form) at the Gauss point
+                  T          nv[3] = {T(0), T(0), T(0)};
                   const bool has_n = a.n[0] != nullptr;
 #pragma unroll
                   for (int l = 0; l < N; ++l)
@@ -94,7 +164,6 @@ namespace mpdg
                         {
                           const int q   = (l * N + j) * N + i;
                           const T   phi = a.B[qx * N + i] * a.B[qy * N + j] * a.B[qz * N + l];
-                          lq += phi * ls[q];
                           if (has_n)
 #pragma unroll
                             for (int d = 0; d < 3; ++d)
@@ -108,8 +177,8 @@ namespace mpdg
                       for (int d = 0; d < 3; ++d)
                         nv[d] *= inv;
                     }
-                  // narrow band: the point contributes only where |level set| < band
-                  const T jw = (a.band_ls && !(fabs(lq) < a.band)) ? T(0) : a.det * a.w[qx] * a.w[qy] * a.w[qz];
+                  const bool in = (bits >> ((qz * N + qy) * N + qx)) & 1u; // narrow band
+                  const T    jw = in ? a.det * a.w[qx] * a.w[qy] * a.w[qz] : T(0);
                   // int phi_i^2 / dt + grad phi_i . D grad phi_i
 #pragma unroll
                   for (int l = 0; l < N; ++l)
@@ -294,74 +363,6 @@ namespace mpdg
       int            mask_src;
     };
 
-    // cell of a lane (a lane outside the mesh reads the fields of the nearest cell), and the values of a
-    // plainly read field at the cell's nodes or Gauss points
-    struct PointCell
-    {
-      int c[3];
-    };
-    template <typename T, int N>
-    __device__ __forceinline__ PointCell
-    point_cell(const GridDesc &g, int cx, int cy, int cz)
-    {
-      return PointCell{{min(cx, g.m[0] - 1), min(cy, g.m[1] - 1), cz}};
-    }
-    template <typename T, int N>
-    __device__ __forceinline__ void
-    field_nodes(const double *f, const GridDesc &g, const PointCell &c, T *v)
-    {
-      constexpr int K  = N - 1;
-      const int     sy = g.n[0], sz = g.n[0] * g.n[1];
-      f += K * c.c[0] + (long long)sy * (K * c.c[1]) + (long long)sz * (K * c.c[2]);
-#pragma unroll
-      for (int l = 0; l < N; ++l)
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-#pragma unroll
-          for (int i = 0; i < N; ++i)
-            v[(l * N + j) * N + i] = (T)__ldg(f + (j * sy + l * sz + i));
-    }
-    template <typename T, int N>
-    __device__ __forceinline__ void
-    interpolate(T *v, const T *B)
-    {
-      gp_interpolate<T, N, 0>(v, B);
-      gp_interpolate<T, N, 1>(v, B);
-      gp_interpolate<T, N, 2>(v, B);
-    }
-    template <typename T, int N>
-    __device__ __forceinline__ void
-    test(T *S, const GaussTab<T, N> &t)
-    {
-      gp_test<T, N, 2>(S, t.Bt[2]);
-      gp_test<T, N, 1>(S, t.Bt[1]);
-      gp_test<T, N, 0>(S, t.Bt[0]);
-    }
-    __device__ __forceinline__ double
-    point_rsqrt(double x)
-    {
-      return rsqrt(x);
-    }
-    __device__ __forceinline__ float
-    point_rsqrt(float x)
-    {
-      return 1.0f / sqrtf(x);
-    }
-    // points of the narrow band, one bit per Gauss point
-    template <typename T, int N, class Args>
-    __device__ __forceinline__ unsigned long long
-    band_bits(const Args &a, const PointCell &c)
-    {
-      T v[N * N * N];
-      field_nodes<T, N>(a.band_ls, a.g, c, v);
-      interpolate<T, N>(v, a.t.B);
-      unsigned long long bits = 0;
-#pragma unroll
-      for (int q = 0; q < N * N * N; ++q)
-        bits |= (unsigned long long)(fabs(v[q]) < a.band ? 1u : 0u) << q;
-      return bits;
-    }
-
     // reinitialisation tangent (RHS = false) and right-hand side (RHS = true: src = psi_old, the flux
     // (1 - psi^2) / 2 n - D grad psi, eps_t and eps with a minus sign), one plane of Gauss points at a time
     template <int K, typename T, bool RHS>
@@ -442,7 +443,7 @@ namespace mpdg
       apply(T *u, const PointCell &c) const
       {
         T                        S[N3];
-        const unsigned long long bits = band_bits<T, N>(a, c);
+        const unsigned long long bits = band_bits<T, N>(a.band_ls, a.band, a.t.B, a.g, c);
         auto in = [&](int q, T x) { return (bits >> q) & 1u ? x : T(0); };
         // u - ref as in ReinitCellOp
         const T ref = u[((K / 2) * N + K / 2) * N + K / 2];
@@ -521,7 +522,7 @@ namespace mpdg
       __device__ __forceinline__ unsigned long long
       band(const PointCell &c) const
       {
-        return a.band_ls ? band_bits<double, N>(a, c) : ~0ull;
+        return a.band_ls ? band_bits<double, N>(a.band_ls, a.band, a.t.B, a.g, c) : ~0ull;
       }
       __device__ __forceinline__ void
       prepare(const MarchNodes<K, double> &nodes, const PointCell &c, State &s) const
@@ -618,7 +619,7 @@ namespace mpdg
           S[q] += v[q];
         if (a.band_ls)
           {
-            const unsigned long long bits = band_bits<double, N>(a, c);
+            const unsigned long long bits = band_bits<double, N>(a.band_ls, a.band, a.t.B, a.g, c);
 #pragma unroll
             for (int q = 0; q < N3; ++q)
               S[q] = (bits >> q) & 1u ? S[q] : 0.0;
@@ -737,7 +738,7 @@ namespace mpdg
       const Tables1D &t = tables(K);
       for (int i = 0; i < N * N; ++i)
         {
-          a.B[i] = (T)t.B[i];
+          a.B[i] = (T)t.ext.B[i]; // as in GaussTab (band_bits)
           a.G[i] = (T)t.G[i];
         }
       for (int q = 0; q < N; ++q)
