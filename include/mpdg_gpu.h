@@ -339,7 +339,8 @@ MPDG_API int mpdg_op_compute_inverse_diagonal_f32(mpdg_op *op, float *diag);
 
 /* OperatorMatrixFree::create_rhs (operator_base.hpp:208-212), accumulating into dst.
    heat (heat_diffuse_operator.cpp:393-529, 783-806):
-     dst += -[(rho c_p/dt)(T - T_old) - q] phi - k grad T . grad phi    (a = T, b = T_old, c = q)
+     dst += -[(rho c_p/dt)(T - T_old) - q] phi - k grad T . grad phi    (a = T, b = T_old, c = q);
+     with constant material dst may share memory with b and c, which are read before anything is added
    advection-diffusion (advection_diffusion_operator.cpp:274-358):
      dst += (u_old/dt - (1-theta) v.grad u_old) phi - (1-theta) eps grad u_old . grad phi (a = u_old) */
 MPDG_API int mpdg_op_create_rhs(mpdg_op *op, double *dst, const double *a, const double *b, const double *c);

@@ -1821,7 +1821,13 @@ mpdg_op_create_rhs(mpdg_op *op, double *dst, const double *a, const double *b, c
     {
       // v = (rho c_p/dt)(T_old - T) + q ; dst += M v - K_k T   (plain reads, free rows)
       const double s = op->rho_cp / op->dt;
-      if (op->degree <= 2 && !op->d_mask && !op->banded())
+      // the one-pass kernel reads T_old and q while it adds to dst; where dst shares memory with one of them the
+      // work vector takes them in before
+      auto apart = [&](const double *x) {
+        const uintptr_t d = reinterpret_cast<uintptr_t>(dst), v = reinterpret_cast<uintptr_t>(x), n = sizeof(double) * op->ndofs;
+        return !x || v + n <= d || d + n <= v;
+      };
+      if (op->degree <= 2 && !op->d_mask && !op->banded() && apart(b) && apart(c))
         {
           HeatLaunch<double> h;
           h.degree = op->degree;
