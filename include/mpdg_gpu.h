@@ -455,7 +455,8 @@ MPDG_API int mpdg_op_device_errors(mpdg_op *op);
    that value on: bricks below it are never processed, so their upper neighbours' waits give up, and
    tickets past the last brick are reported and skipped.  The last CTA of that launch resets the
    counter, so later launches are normal again.
-   mpdg_op_n_bricks: bricks of the handle's FP64 apply (the range of useful ticket values). */
+   mpdg_op_n_bricks: the range of useful ticket values: bricks that every FP64 apply of the handle as it is
+   set up now has at least (the bricks of full height, or the launch's own where it cuts z into fewer). */
 MPDG_API int mpdg_op_test_set_wait_limit(mpdg_op *op, unsigned spins);
 /* Selects the implementation of the Jacobi-CG iteration behind mpdg_solve / mpdg_solve_f32 / the
    inner solves of mpdg_solve_mixed (LinearSolver::solve with SolverCG, linear_solver.hpp:106-110):

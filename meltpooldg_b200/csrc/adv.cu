@@ -483,6 +483,21 @@ namespace mpdg
     return std::max(march_flags(m, sd[2]), march_flags(m, sf[2]));
   }
 
+  template <int K>
+  static long long
+  launch_bricks(const int m[3], bool supg, bool field)
+  {
+    return march_bricks(m, MarchShape<K, double>::BZ,
+                        supg ? (field ? AdvMinBlocks<K, double, true, true>::value : AdvMinBlocks<K, double, true, false>::value) :
+                               (field ? AdvMinBlocks<K, double, false, true>::value : AdvMinBlocks<K, double, false, false>::value));
+  }
+
+  long long
+  adv_launch_bricks(int K, const int m[3], bool supg, bool field)
+  {
+    return K == 1 ? launch_bricks<1>(m, supg, field) : (K == 2 ? launch_bricks<2>(m, supg, field) : launch_bricks<3>(m, supg, field));
+  }
+
   // ---- diagonal in closed form (MatrixFreeTools::compute_diagonal of the tangent).
   // With phi_i = phi_a(x) phi_b(y) phi_c(z) and an affine velocity, every term of
   //   A_ii = int phi_i^2 / dt + theta v . grad(phi_i) phi_i + theta eps |grad phi_i|^2

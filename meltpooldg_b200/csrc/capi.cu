@@ -2350,7 +2350,18 @@ mpdg_op_n_bricks(const mpdg_op *op)
 {
   if (!op)
     return -1;
-  return op->nbr[0] * op->nbr[1] * op->nbr[2];
+  // the applies choose their own cut in z; the value is one that no FP64 apply of the handle goes below
+  const long long full = (long long)op->nbr[0] * op->nbr[1] * op->nbr[2];
+  long long       n    = full;
+  if (op->kind == MPDG_REINIT || op->banded())
+    n = reinit_launch_bricks(op->degree, op->m, op->banded());
+  else if (op->kind == MPDG_HEAT && op->solid)
+    n = heat_solid_launch_bricks(op->degree, op->m);
+  else if (op->kind == MPDG_ADVDIFF || op->d_vfield[0])
+    n = adv_launch_bricks(op->degree, op->m, op->kind == MPDG_ADVDIFF && op->supg, op->d_vfield[0] != nullptr);
+  else
+    n = heat_launch_bricks(op->degree, op->m, op->d_mask == nullptr);
+  return (int)std::min(full, n);
 }
 
 int

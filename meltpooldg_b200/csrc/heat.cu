@@ -867,6 +867,30 @@ namespace mpdg
     return march ? std::max(most, PENCIL_MIN_FLAGS) : most;
   }
 
+  template <int K>
+  static long long
+  pencil_bricks(const int m[3])
+  {
+    using S = PencilShape<K>;
+    return (long long)((m[0] + S::BX - 1) / S::BX) * ((m[1] + S::BY - 1) / S::BY) * pencil_plan(m, S::BX, S::BY, S::BZ, 148 * S::MINB);
+  }
+
+  long long
+  heat_launch_bricks(int K, const int m[3], bool march)
+  {
+    if (march)
+      switch (K)
+        {
+          case 1: return march_bricks(m, MarchShape<1, double>::BZ, MarchMinBlocks<1, double>::value);
+          case 2: return march_bricks(m, MarchShape<2, double>::BZ, MarchMinBlocks<2, double>::value);
+          case 3: return pencil_bricks<3>(m);
+          default: return pencil_bricks<4>(m);
+        }
+    int sh[3];
+    heat_brick_shape<double>(K, sh, false);
+    return (long long)((m[0] + sh[0] - 1) / sh[0]) * ((m[1] + sh[1] - 1) / sh[1]) * ((m[2] + sh[2] - 1) / sh[2]);
+  }
+
   template <int K, typename T>
   static cudaError_t
   dispatch_mode(const HeatLaunch<T> &h, cudaStream_t s)

@@ -492,6 +492,14 @@ namespace mpdg
     }
   } // namespace
 
+  long long
+  heat_solid_launch_bricks(int K, const int m[3])
+  {
+    return K == 1 ? march_bricks(m, MarchShape<1, double>::BZ, SolidMinBlocks<1, double>::value) :
+                    (K == 2 ? march_bricks(m, MarchShape<2, double>::BZ, SolidMinBlocks<2, double>::value) :
+                              march_bricks(m, MarchShape<3, double>::BZ, SolidMinBlocks<3, double>::value));
+  }
+
   template <typename T>
   cudaError_t
   heat_solid_apply(const HeatSolidLaunch<T> &h, cudaStream_t s)

@@ -55,6 +55,8 @@ namespace mpdg
   void heat_brick_shape(int K, int shape[3], bool march);
   // init flags (and fused-dot partials) that an apply of this mesh may use, in either precision
   long long heat_flags(int K, const int m[3], bool march);
+  // bricks that the FP64 apply launches
+  long long heat_launch_bricks(int K, const int m[3], bool march);
 
   // ---- boundary-face terms of the heat operator (faces.cu); face f: bit 2d low / 2d+1 high of dim d
   struct HeatFaceBC
@@ -115,6 +117,7 @@ namespace mpdg
 
   template <typename T>
   cudaError_t heat_solid_apply(const HeatSolidLaunch<T> &h, cudaStream_t s);
+  long long   heat_solid_launch_bricks(int K, const int m[3]);
   // diag = the tangent's diagonal (FP64), constrained rows 0
   cudaError_t heat_solid_diagonal(const GridDesc &g, const SyncDesc &sync, int K, const SolidMaterial &mat, double dt,
                                   const double hlen[3], const double *temp, const double *temp_old, double *diag,
@@ -144,6 +147,7 @@ namespace mpdg
   // on free rows
   template <typename T>
   cudaError_t reinit_integrate(const ReinitLaunch<T> &h, int mode, cudaStream_t s);
+  long long   reinit_launch_bricks(int K, const int m[3], bool banded);
   // normal-vector (mode 0: out_d += int grad_d psi phi, normalised on request) and curvature (mode 1:
   // out0 = -int div(normalize(n_i, tol)) phi, constrained rows 0) right-hand sides, FE_Q(1..3)
   // band_ls / band: optional narrow band (integrand masked where |band_ls(x_q)| >= band)
@@ -204,6 +208,7 @@ namespace mpdg
   void adv_brick_shape(int K, int shape[3]);
   // init flags that an advection-form apply of this mesh may use, in either precision
   long long adv_flags(int K, const int m[3]);
+  long long adv_launch_bricks(int K, const int m[3], bool supg, bool field);
 
   // ---- vectors and reductions (double accumulation for every vector type)
   constexpr int RED_BLOCKS  = 592; // 4 x 148 SMs

@@ -89,6 +89,15 @@ namespace mpdg
     return (unsigned)g.nbr[0] * g.nbr[1] * g.nbr[2];
   }
 
+  inline long long
+  march_bricks(const int m[3], int bz_full, int per_sm)
+  {
+    GridDesc g{};
+    for (int d = 0; d < 3; ++d)
+      g.m[d] = m[d];
+    return march_grid(g, bz_full, per_sm);
+  }
+
   // flags / dot partials an operator must hold for the segments of any of its marching applies
   inline long long
   march_flags(const int m[3], int bz_full)

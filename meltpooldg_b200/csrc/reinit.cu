@@ -861,6 +861,21 @@ namespace mpdg
       }
   }
 
+  template <int K>
+  static long long
+  launch_bricks(const int m[3], bool banded)
+  {
+    return march_bricks(m, MarchShape<K, double>::BZ,
+                        banded ? PointMinBlocks<K, double, BandCellOp<K, double>::HEAVY>::value :
+                                 PointMinBlocks<K, double, ReinitCellOp<K, double, false>::HEAVY>::value);
+  }
+
+  long long
+  reinit_launch_bricks(int K, const int m[3], bool banded)
+  {
+    return K == 1 ? launch_bricks<1>(m, banded) : (K == 2 ? launch_bricks<2>(m, banded) : launch_bricks<3>(m, banded));
+  }
+
   template <typename T>
   cudaError_t
   reinit_integrate(const ReinitLaunch<T> &h, int mode, cudaStream_t s)
