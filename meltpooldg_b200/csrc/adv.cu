@@ -351,7 +351,7 @@ namespace mpdg
                                  K == 2 ? (SUPG && VDOF ? 2 : SUPG ? (f64 ? 2 : 4) : VDOF ? (f64 ? 2 : 3) : (f64 ? 3 : 5)) : 2;
   };
 
-  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF>
+  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF, int BX>
   __global__ void __launch_bounds__(MARCH_NT, AdvMinBlocks<K, T, SUPG, VDOF>::value)
   adv_apply_kernel(const __grid_constant__ AdvArgs<T, K + 1> a)
   {
@@ -361,22 +361,32 @@ namespace mpdg
     if (a.skip != nullptr && *a.skip != 0)
       return;
     AdvCellOp<K, T, SUPG, VDOF> op{a};
-    march_body<K, T, MODE, AdvCellOp<K, T, SUPG, VDOF>, false, true>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
+    march_body<K, T, MODE, AdvCellOp<K, T, SUPG, VDOF>, false, true, BX>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
                                                                      reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
+  }
+
+  template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF, int BX>
+  static cudaError_t
+  launch_adv_columns(AdvArgs<T, K + 1> &a, cudaStream_t stream)
+  {
+    auto                                   kern = adv_apply_kernel<K, T, MODE, SUPG, VDOF, BX>;
+    static std::atomic<unsigned long long> devices{0};
+    constexpr size_t                       bytes = MarchLayout<K, T, BX>::bytes;
+    if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
+      return e;
+    const unsigned ctas = march_grid(a.g, BX, MarchShape<K, T>::BZ, AdvMinBlocks<K, T, SUPG, VDOF>::value);
+    kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
+    return cudaGetLastError();
   }
 
   template <int K, typename T, OutMode MODE, bool SUPG, bool VDOF>
   static cudaError_t
   launch_adv_kernel(AdvArgs<T, K + 1> &a, cudaStream_t stream)
   {
-    auto                                   kern = adv_apply_kernel<K, T, MODE, SUPG, VDOF>;
-    static std::atomic<unsigned long long> devices{0};
-    constexpr size_t                       bytes = MarchLayout<K, T>::bytes;
-    if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
-      return e;
-    const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, AdvMinBlocks<K, T, SUPG, VDOF>::value);
-    kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
-    return cudaGetLastError();
+    if constexpr (MODE != OutMode::BPlus) // b + A x is formed once a solve: one width
+      if (march_bx(a.g.m) != MARCH_BX)
+        return launch_adv_columns<K, T, MODE, SUPG, VDOF, MARCH_BX_NARROW>(a, stream);
+    return launch_adv_columns<K, T, MODE, SUPG, VDOF, MARCH_BX>(a, stream);
   }
 
   template <int K, typename T, OutMode MODE>
@@ -470,24 +480,23 @@ namespace mpdg
   adv_brick_shape(int K, int shape[3])
   {
     shape[0] = MARCH_BX;
-    shape[1] = MARCH_BY;
+    shape[1] = MARCH_NT / MARCH_BX;
     shape[2] = K == 1 ? MarchShape<1, T>::BZ : (K == 2 ? MarchShape<2, T>::BZ : MarchShape<3, T>::BZ);
   }
 
   long long
   adv_flags(int K, const int m[3])
   {
-    int sd[3], sf[3];
-    adv_brick_shape<double>(K, sd);
-    adv_brick_shape<float>(K, sf);
-    return std::max(march_flags(m, sd[2]), march_flags(m, sf[2]));
+    int shape[3]; // FP64: the shorter full-length segments
+    adv_brick_shape<double>(K, shape);
+    return std::max(march_flags(m, MARCH_BX, shape[2]), march_flags(m, march_bx(m), shape[2]));
   }
 
   template <int K>
   static long long
   launch_bricks(const int m[3], bool supg, bool field)
   {
-    return march_bricks(m, MarchShape<K, double>::BZ,
+    return march_bricks(m, march_bx(m), MarchShape<K, double>::BZ,
                         supg ? (field ? AdvMinBlocks<K, double, true, true>::value : AdvMinBlocks<K, double, true, false>::value) :
                                (field ? AdvMinBlocks<K, double, false, true>::value : AdvMinBlocks<K, double, false, false>::value));
   }

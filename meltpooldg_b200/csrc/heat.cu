@@ -710,7 +710,7 @@ namespace mpdg
       if (h.grid.cmask == nullptr && h.march)
         {
           using ML = MarchLayout<K, T>;
-          const unsigned nbricks = march_grid(a.g, MarchShape<K, T>::BZ, MarchMinBlocks<K, T>::value);
+          const unsigned nbricks = march_grid(a.g, MARCH_BX, MarchShape<K, T>::BZ, MarchMinBlocks<K, T>::value);
           static std::atomic<unsigned long long> dev_plain{0}, dev_dot{0};
           if constexpr (MODE == OutMode::Set)
             if (h.dot.part != nullptr)
@@ -794,7 +794,7 @@ namespace mpdg
     constexpr size_t                       bytes = MarchLayout<K, double>::bytes;
     if ((e = ensure_smem(kern, bytes, devices)) != cudaSuccess)
       return e;
-    const unsigned ctas = march_grid(r.a.g, MarchShape<K, double>::BZ, heat_rhs_minb(K));
+    const unsigned ctas = march_grid(r.a.g, MARCH_BX, MarchShape<K, double>::BZ, heat_rhs_minb(K));
     kern<<<ctas, MARCH_NT, bytes, stream>>>(r);
     return cudaGetLastError();
   }
@@ -816,8 +816,8 @@ namespace mpdg
   {
     switch (K)
       {
-        case 1: bx = MarchShape<1, T>::BX; by = MarchShape<1, T>::BY; bz = MarchShape<1, T>::BZ; break;
-        case 2: bx = MarchShape<2, T>::BX; by = MarchShape<2, T>::BY; bz = MarchShape<2, T>::BZ; break;
+        case 1: bx = MARCH_BX; by = MARCH_NT / MARCH_BX; bz = MarchShape<1, T>::BZ; break;
+        case 2: bx = MARCH_BX; by = MARCH_NT / MARCH_BX; bz = MarchShape<2, T>::BZ; break;
         case 3: bx = HeatBrickShape<3, T>::BX; by = HeatBrickShape<3, T>::BY; bz = HeatBrickShape<3, T>::BZ; break;
         default: bx = HeatBrickShape<4, T>::BX; by = HeatBrickShape<4, T>::BY; bz = HeatBrickShape<4, T>::BZ; break;
       }
@@ -849,8 +849,8 @@ namespace mpdg
   heat_flags(int K, const int m[3], bool march)
   {
     if (march && K <= 2)
-      return std::max(march_flags(m, K == 1 ? MarchShape<1, double>::BZ : MarchShape<2, double>::BZ),
-                      march_flags(m, K == 1 ? MarchShape<1, float>::BZ : MarchShape<2, float>::BZ));
+      return std::max(march_flags(m, MARCH_BX, K == 1 ? MarchShape<1, double>::BZ : MarchShape<2, double>::BZ),
+                      march_flags(m, MARCH_BX, K == 1 ? MarchShape<1, float>::BZ : MarchShape<2, float>::BZ));
     long long most = 1;
     for (int prec = 0; prec < 2; ++prec)
       {
@@ -881,8 +881,8 @@ namespace mpdg
     if (march)
       switch (K)
         {
-          case 1: return march_bricks(m, MarchShape<1, double>::BZ, MarchMinBlocks<1, double>::value);
-          case 2: return march_bricks(m, MarchShape<2, double>::BZ, MarchMinBlocks<2, double>::value);
+          case 1: return march_bricks(m, MARCH_BX, MarchShape<1, double>::BZ, MarchMinBlocks<1, double>::value);
+          case 2: return march_bricks(m, MARCH_BX, MarchShape<2, double>::BZ, MarchMinBlocks<2, double>::value);
           case 3: return pencil_bricks<3>(m);
           default: return pencil_bricks<4>(m);
         }

@@ -362,7 +362,7 @@ namespace mpdg
       static constexpr int value = MPDG_SOLID_MINB ? MPDG_SOLID_MINB : K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? 3 : 4) : 2);
     };
 
-    template <int K, typename T, OutMode MODE, class Op>
+    template <int K, typename T, OutMode MODE, class Op, int BX>
     __global__ void __launch_bounds__(MARCH_NT, SolidMinBlocks<K, T>::value)
     heat_solid_kernel(const __grid_constant__ SolidArgs<T, K + 1> a)
     {
@@ -372,7 +372,7 @@ namespace mpdg
       if (a.skip != nullptr && *a.skip != 0)
         return;
       Op op{a};
-      march_body<K, T, MODE, Op, false, true>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
+      march_body<K, T, MODE, Op, false, true, BX>(a.g, a.s, a.src, a.dst, a.b, a.mask_src != 0, op,
                                               reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
     }
 
@@ -403,18 +403,28 @@ namespace mpdg
       return s;
     }
 
+    template <int K, typename T, OutMode MODE, class Op, int BX>
+    cudaError_t
+    launch_solid_columns(SolidArgs<T, K + 1> &a, cudaStream_t stream)
+    {
+      auto                                   kern = heat_solid_kernel<K, T, MODE, Op, BX>;
+      static std::atomic<unsigned long long> devices{0};
+      constexpr size_t                       bytes = MarchLayout<K, T, BX>::bytes;
+      if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
+        return e;
+      const unsigned ctas = march_grid(a.g, BX, MarchShape<K, T>::BZ, SolidMinBlocks<K, T>::value);
+      kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
+      return cudaGetLastError();
+    }
+
     template <int K, typename T, OutMode MODE, class Op>
     cudaError_t
     launch_solid(SolidArgs<T, K + 1> &a, cudaStream_t stream)
     {
-      auto                                   kern = heat_solid_kernel<K, T, MODE, Op>;
-      static std::atomic<unsigned long long> devices{0};
-      constexpr size_t                       bytes = MarchLayout<K, T>::bytes;
-      if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
-        return e;
-      const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, SolidMinBlocks<K, T>::value);
-      kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
-      return cudaGetLastError();
+      if constexpr (MODE != OutMode::BPlus) // b + A x is formed once a solve: one width
+        if (march_bx(a.g.m) != MARCH_BX)
+          return launch_solid_columns<K, T, MODE, Op, MARCH_BX_NARROW>(a, stream);
+      return launch_solid_columns<K, T, MODE, Op, MARCH_BX>(a, stream);
     }
 
     template <int K, typename T>
@@ -495,9 +505,9 @@ namespace mpdg
   long long
   heat_solid_launch_bricks(int K, const int m[3])
   {
-    return K == 1 ? march_bricks(m, MarchShape<1, double>::BZ, SolidMinBlocks<1, double>::value) :
-                    (K == 2 ? march_bricks(m, MarchShape<2, double>::BZ, SolidMinBlocks<2, double>::value) :
-                              march_bricks(m, MarchShape<3, double>::BZ, SolidMinBlocks<3, double>::value));
+    return K == 1 ? march_bricks(m, march_bx(m), MarchShape<1, double>::BZ, SolidMinBlocks<1, double>::value) :
+                    (K == 2 ? march_bricks(m, march_bx(m), MarchShape<2, double>::BZ, SolidMinBlocks<2, double>::value) :
+                              march_bricks(m, march_bx(m), MarchShape<3, double>::BZ, SolidMinBlocks<3, double>::value));
   }
 
   template <typename T>

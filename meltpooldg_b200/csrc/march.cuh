@@ -33,7 +33,7 @@
 
 namespace mpdg
 {
-  constexpr int MARCH_BX = 32, MARCH_BY = 4, MARCH_NT = 128;
+  constexpr int MARCH_BX = 32, MARCH_BX_NARROW = 16, MARCH_NT = 128;
   // segments of any mesh: at most the full-length ones or this many (brick flags, dot partials)
   constexpr long long MARCH_MIN_FLAGS = 8192;
 
@@ -42,9 +42,30 @@ namespace mpdg
   template <int K, typename T>
   struct MarchShape
   {
-    static constexpr int BX = MARCH_BX, BY = MARCH_BY, NT = MARCH_NT;
     static constexpr int BZ = K == 1 ? 16 : (sizeof(T) == 4 ? 16 : 8);
   };
+
+  inline long long
+  march_columns(const int m[3], int bx)
+  {
+    const int by = MARCH_NT / bx;
+    return (long long)((m[0] + bx - 1) / bx) * ((m[1] + by - 1) / by);
+  }
+
+  // Column width of the operators with coefficients inside the cells (the heat apply always takes 32 x 4): 16 x 8
+  // cells where they leave at most 4/5 of the threads that 32 x 4 cells take and the mesh fills the chip (two CTAs
+  // per SM in segments of one layer).  A row of lanes outside the mesh costs as much as one inside: FE_Q(3) FP64
+  // 48^3 (3/4) temperature-dependent tangent 360 -> 303 us, advection 70 -> 56, reinitialisation 315 -> 262;
+  // FE_Q(1) 8x40x160 (1/2) advection 14.5 -> 11.3, tangent 28.9 -> 21.2.  At 5/6 the wider column still wins on
+  // small meshes (FE_Q(2) 33x33x40 reinitialisation 43 against 48 us), at equal counts by up to 5 % (FE_Q(1)
+  // 192x160x72 advection 71.6 against 74.1), and where a launch takes one CTA's time by its shorter chain, half as many
+  // rows to stage (FE_Q(2) 12^3, 2/3: reinitialisation 16.5 against 17.5, banded FP32 10.4 against 12.3).
+  inline int
+  march_bx(const int m[3])
+  {
+    const long long wide = march_columns(m, MARCH_BX);
+    return 5 * march_columns(m, MARCH_BX_NARROW) <= 4 * wide && wide * m[2] >= 2 * 148 ? MARCH_BX_NARROW : MARCH_BX;
+  }
 
   // Segment length for a mesh: the bz whose CTAs take the least time on the resident slots.  In units of
   // a layer at full occupancy a CTA costs its layers plus about one (two, where it starts on an idle
@@ -54,9 +75,9 @@ namespace mpdg
   // full wave) against 88 at 8 (864 segments on 740 slots) and 81 at 16; 64^3 25 us at 3 against 36 at
   // 8; 32^3 10 us at 1 against 33 at 8.
   inline int
-  march_plan(const int m[3], int bz_full, int slots, int *nseg)
+  march_plan(const int m[3], int bx, int bz_full, int slots, int *nseg)
   {
-    const long long cols = (long long)((m[0] + MARCH_BX - 1) / MARCH_BX) * ((m[1] + MARCH_BY - 1) / MARCH_BY);
+    const long long cols = march_columns(m, bx);
     const long long cap  = cols * ((m[2] + bz_full - 1) / bz_full);
     double          best = 0.0;
     int             bz   = bz_full;
@@ -81,45 +102,44 @@ namespace mpdg
   // The column counts and the segment length of a launch on 148 SMs with per_sm resident CTAs; returns
   // the number of CTAs.
   inline unsigned
-  march_grid(GridDesc &g, int bz_full, int per_sm)
+  march_grid(GridDesc &g, int bx, int bz_full, int per_sm)
   {
-    g.nbr[0] = (g.m[0] + MARCH_BX - 1) / MARCH_BX;
-    g.nbr[1] = (g.m[1] + MARCH_BY - 1) / MARCH_BY;
-    g.bz     = march_plan(g.m, bz_full, 148 * per_sm, &g.nbr[2]);
+    g.nbr[0] = (g.m[0] + bx - 1) / bx;
+    g.nbr[1] = (g.m[1] + MARCH_NT / bx - 1) / (MARCH_NT / bx);
+    g.bz     = march_plan(g.m, bx, bz_full, 148 * per_sm, &g.nbr[2]);
     return (unsigned)g.nbr[0] * g.nbr[1] * g.nbr[2];
   }
 
   inline long long
-  march_bricks(const int m[3], int bz_full, int per_sm)
+  march_bricks(const int m[3], int bx, int bz_full, int per_sm)
   {
     GridDesc g{};
     for (int d = 0; d < 3; ++d)
       g.m[d] = m[d];
-    return march_grid(g, bz_full, per_sm);
+    return march_grid(g, bx, bz_full, per_sm);
   }
 
   // flags / dot partials an operator must hold for the segments of any of its marching applies
   inline long long
-  march_flags(const int m[3], int bz_full)
+  march_flags(const int m[3], int bx, int bz_full)
   {
-    const long long cols = (long long)((m[0] + MARCH_BX - 1) / MARCH_BX) * ((m[1] + MARCH_BY - 1) / MARCH_BY);
-    const long long cap  = cols * ((m[2] + bz_full - 1) / bz_full);
+    const long long cap = march_columns(m, bx) * ((m[2] + bz_full - 1) / bz_full);
     return cap > MARCH_MIN_FLAGS ? cap : MARCH_MIN_FLAGS;
   }
 
-  template <int K, typename T>
+  template <int K, typename T, int BX = MARCH_BX>
   struct MarchLayout
   {
-    static constexpr int N = K + 1, G = 16 / (int)sizeof(T);
-    static constexpr int PX = K * MARCH_BX + 1, PY = K * MARCH_BY + 1, NRING = 2 * K + 1;
+    static constexpr int N = K + 1, G = 16 / (int)sizeof(T), BY = MARCH_NT / BX;
+    static constexpr int PX = K * BX + 1, PY = K * BY + 1, NRING = 2 * K + 1;
     static constexpr int PITCH = (PX + G - 1 + G - 1) / G * G; // row of a slot: shift + points
     static constexpr int PLANE = PY * PITCH;
-    static constexpr int YX    = MARCH_BY * N * K * 32;        // y-exchange, one buffer
+    static constexpr int YX    = N * K * MARCH_NT;             // y-exchange, one buffer
     static constexpr size_t bytes = sizeof(T) * (NRING * (size_t)PLANE + 2 * (size_t)YX);
   };
 
   // Geometry of one column segment (K points per cell; bz layers)
-  template <int K>
+  template <int K, int BX>
   struct Column
   {
     int      c0[3], g0[3], nv[3];
@@ -130,9 +150,9 @@ namespace mpdg
     set(const GridDesc &g, unsigned t)
     {
       id           = t;
-      const int B[3] = {MARCH_BX, MARCH_BY, g.bz};
-      c0[0]        = (int)(t % (unsigned)g.nbr[0]) * MARCH_BX;
-      c0[1]        = (int)((t / (unsigned)g.nbr[0]) % (unsigned)g.nbr[1]) * MARCH_BY;
+      const int B[3] = {BX, MARCH_NT / BX, g.bz};
+      c0[0]        = (int)(t % (unsigned)g.nbr[0]) * B[0];
+      c0[1]        = (int)((t / (unsigned)g.nbr[0]) % (unsigned)g.nbr[1]) * B[1];
       c0[2]        = (int)(t / (unsigned)(g.nbr[0] * g.nbr[1])) * g.bz;
       any_con      = 0;
 #pragma unroll
@@ -165,9 +185,9 @@ namespace mpdg
   // Initialise the face points the segment owns (Set: 0, BPlus: b) and publish the flag: its high faces
   // and, at the domain's low boundary, its low faces (edge points are visited up to three times with the
   // same value).  acc_lo_z: the lattice's low z plane holds the previous slab's values and stays.
-  template <int K, typename T, OutMode MODE>
+  template <int K, typename T, OutMode MODE, int BX>
   __device__ __forceinline__ void
-  column_init_publish(const Column<K> &br, const SyncDesc &s, T *dst, const T *bvec, unsigned acc_lo_z)
+  column_init_publish(const Column<K, BX> &br, const SyncDesc &s, T *dst, const T *bvec, unsigned acc_lo_z)
   {
     static_assert(MODE != OutMode::Add, "Add mode needs no initialisation");
     auto put = [&](int px, int py, int pz) {
@@ -178,12 +198,14 @@ namespace mpdg
       const int idx = br.index(px, py, pz);
       dst[idx]      = (MODE == OutMode::BPlus) ? bvec[idx] : T(0);
     };
-    constexpr int PX = K * MARCH_BX + 1;
+    constexpr int PX = K * BX + 1, PY = K * (MARCH_NT / BX) + 1;
     const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int side = br.lo_sh[0] ? 1 : 0; side < 2; ++side)
       for (int pz = warp; pz < br.nv[2]; pz += MARCH_NT / 32)
-        if (lane < br.nv[1])
-          put(side ? br.nv[0] - 1 : 0, lane, pz);
+#pragma unroll
+        for (int c = 0; c < (PY + 31) / 32; ++c)
+          if (lane + 32 * c < br.nv[1])
+            put(side ? br.nv[0] - 1 : 0, lane + 32 * c, pz);
     for (int side = br.lo_sh[1] ? 1 : 0; side < 2; ++side)
       for (int pz = warp; pz < br.nv[2]; pz += MARCH_NT / 32)
 #pragma unroll
@@ -206,9 +228,9 @@ namespace mpdg
 
   // Bounded wait of threads 0..6 for the flags of the lower neighbour segments; the caller's next
   // barrier orders the other threads.
-  template <int K>
+  template <int K, int BX>
   __device__ __forceinline__ void
-  column_wait_lower(const Column<K> &br, const GridDesc &g, const SyncDesc &s)
+  column_wait_lower(const Column<K, BX> &br, const GridDesc &g, const SyncDesc &s)
   {
     if (threadIdx.x < 7)
       {
@@ -299,11 +321,11 @@ namespace mpdg
 
   // Warp 0: the planes [p0, p1) of the segment into their ring slots (slot = plane mod NRING); every
   // lane arrives on the barrier once (count 32), with the bytes of its rows.
-  template <int K, typename T>
+  template <int K, typename T, int BX>
   __device__ __forceinline__ void
-  march_stage(const Column<K> &br, const T *src, int n_src, int base, int p0, int p1, T *ring, unsigned long long *bar)
+  march_stage(const Column<K, BX> &br, const T *src, int n_src, int base, int p0, int p1, T *ring, unsigned long long *bar)
   {
-    using LAY = MarchLayout<K, T>;
+    using LAY = MarchLayout<K, T, BX>;
     const int lane = threadIdx.x;
     const int rows = (p1 - p0) * LAY::PY;
     auto      row  = [&](int r, bool issue) -> unsigned {
@@ -366,18 +388,18 @@ namespace mpdg
   // An operator with Op::OUT results (NODES) has op.prepare(nodes, pre, state), op.component<m>(u, nodes, state)
   // and the output vectors op.out(m) instead: result after result of a layer is exchanged and written.
   // MASKABLE: the operator may carry per-DoF constraint flags (GridDesc::cmask) besides the faces.
-  template <int K, typename T, OutMode MODE, class Op, bool DOT = false, bool MASKABLE = false>
+  template <int K, typename T, OutMode MODE, class Op, bool DOT = false, bool MASKABLE = false, int BX = MARCH_BX>
   __device__ __forceinline__ void
   march_body(const GridDesc &g, const SyncDesc &s, const T *src, T *dst, const T *bvec, bool mask_src, const Op &op,
              T *smem, unsigned *s_ticket, unsigned long long *bars, const DotSink &dot = DotSink{},
              double *s_red = nullptr)
   {
     double dsum = 0.0;
-    using LAY   = MarchLayout<K, T>;
+    using LAY   = MarchLayout<K, T, BX>;
     constexpr int N = K + 1, G = LAY::G, PITCH = LAY::PITCH, NRING = LAY::NRING;
     T *ring = smem, *yx0 = smem + NRING * LAY::PLANE;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Column<K> br;
+    const int     lx = threadIdx.x % BX, row = threadIdx.x / BX; // the thread's cell in the column
+    Column<K, BX> br;
     if (threadIdx.x == 0)
       {
         march_bar_init(&bars[0], 32);
@@ -405,18 +427,18 @@ namespace mpdg
     const int n_src = g.n[0] * g.n[1] * g.n[2];
     const int base  = (int)((reinterpret_cast<unsigned long long>(src) / sizeof(T)) & (G - 1));
     const int nlayers = br.layers;
-    if (warp == 0)
+    if (row < 32 / BX) // warp 0
       {
-        march_stage<K, T>(br, src, n_src, base, 0, K + 1, ring, &bars[0]);
+        march_stage<K, T, BX>(br, src, n_src, base, 0, K + 1, ring, &bars[0]);
         if (nlayers > 1)
-          march_stage<K, T>(br, src, n_src, base, K + 1, 2 * K + 1, ring, &bars[1]);
+          march_stage<K, T, BX>(br, src, n_src, base, K + 1, 2 * K + 1, ring, &bars[1]);
       }
     if constexpr (MODE != OutMode::Add)
-      column_init_publish<K, T, MODE>(br, s, dst, bvec, g.acc_lo_z);
-    const int  cx = br.c0[0] + lane, cy = br.c0[1] + warp;
+      column_init_publish<K, T, MODE, BX>(br, s, dst, bvec, g.acc_lo_z);
+    const int  cx = br.c0[0] + lx, cy = br.c0[1] + row;
     const bool vxy       = cx < g.m[0] && cy < g.m[1];
-    const bool last_lane = cx == min(br.c0[0] + MARCH_BX, g.m[0]) - 1;
-    const bool last_warp = cy == min(br.c0[1] + MARCH_BY, g.m[1]) - 1;
+    const bool x_last = cx == min(br.c0[0] + BX, g.m[0]) - 1;
+    const bool y_last = cy == min(br.c0[1] + LAY::BY, g.m[1]) - 1;
     const bool do_mask   = mask_src && br.any_con; // only segments on a constrained face pay for masking
     // Dirichlet planes through the cell
     const bool cI0 = br.con_lo[0] && cx == 0, cIK = br.con_hi[0] && cx == g.m[0] - 1;
@@ -428,7 +450,7 @@ namespace mpdg
 #pragma unroll
       for (int q = 0; q < K * K; ++q)
         carry[m][q] = T(0);
-    const int wbase  = br.index(0, K * warp, 0); // first point of the warp's cell row
+    const int wbase  = br.index(0, K * row, 0); // first point of the cell row
     int       slot0  = 0;                          // ring slot of the layer's low plane
     for (int lz = 0; lz < nlayers; ++lz)
       {
@@ -436,7 +458,7 @@ namespace mpdg
         // warps outside the mesh, too
         const int  cz  = br.c0[2] + lz;
         const auto pre = op.load(vxy, cx, cy, cz); // per-cell coefficients, in flight during the wait
-        if (!march_bar_wait(&bars[lz & 1], (unsigned)(lz >> 1) & 1u) && lane == 0)
+        if (!march_bar_wait(&bars[lz & 1], (unsigned)(lz >> 1) & 1u) && lx == 0)
           atomicExch(s.error, ERR_FLAG_WAIT);
         const bool last_layer = lz == nlayers - 1;
         const bool cL0 = br.con_lo[2] && cz == 0, cLK = br.con_hi[2] && cz == g.m[2] - 1;
@@ -449,7 +471,7 @@ namespace mpdg
             int sl = slot0 + l;
             if (sl >= NRING)
               sl -= NRING;
-            const T  *pl = ring + sl * LAY::PLANE + (K * warp) * PITCH + K * lane;
+            const T  *pl = ring + sl * LAY::PLANE + (K * row) * PITCH + K * lx;
             const int e  = base + wbase + br.sz * (K * lz + l);
 #pragma unroll
             for (int j = 0; j < N; ++j)
@@ -460,34 +482,34 @@ namespace mpdg
           slot0 -= NRING;
         // exchange of result m (u) with the neighbouring cells and write-out to out
         auto finish = [&](const int m, T *out) {
-          // x: lane t adds lane t-1's x = K face
+          // x: a cell adds its lower neighbour's x = K face
 #pragma unroll
           for (int q = 0; q < N * N; ++q)
             {
               const T v = __shfl_up_sync(0xffffffffu, u[q * N + K], 1);
-              if (lane > 0)
+              if (lx > 0)
                 u[q * N] += v;
             }
-          // y: warp w hands its y = K face to warp w + 1 (the last warp adds its own to dst below)
+          // y: a cell row hands its y = K face to the next (the last adds its own to dst below)
           T *yx = yx0 + ((OUT * lz + m) & 1) * LAY::YX;
 #pragma unroll
           for (int l = 0; l < N; ++l)
 #pragma unroll
             for (int i = 0; i < K; ++i)
-              yx[((warp * N + l) * K + i) * 32 + lane] = u[(l * N + K) * N + i];
+              yx[((row * N + l) * K + i) * BX + lx] = u[(l * N + K) * N + i];
           if constexpr (MODE != OutMode::Add)
             if (lz == 0 && m == 0 && br.has_lower_neighbour())
-              column_wait_lower<K>(br, g, s);
+              column_wait_lower<K, BX>(br, g, s);
           __syncthreads();
           // every thread has read the layer's planes: those that the layer after next needs not are free
-          if (m == OUT - 1 && warp == 0 && lz + 2 < nlayers)
-            march_stage<K, T>(br, src, n_src, base, K * (lz + 2) + 1, K * (lz + 3) + 1, ring, &bars[lz & 1]);
-          if (warp > 0)
+          if (m == OUT - 1 && row < 32 / BX && lz + 2 < nlayers)
+            march_stage<K, T, BX>(br, src, n_src, base, K * (lz + 2) + 1, K * (lz + 3) + 1, ring, &bars[lz & 1]);
+          if (row > 0)
 #pragma unroll
             for (int l = 0; l < N; ++l)
 #pragma unroll
               for (int i = 0; i < K; ++i)
-                u[(l * N) * N + i] += yx[(((warp - 1) * N + l) * K + i) * 32 + lane];
+                u[(l * N) * N + i] += yx[(((row - 1) * N + l) * K + i) * BX + lx];
           // z: add the carried face, carry this layer's z = K face
 #pragma unroll
           for (int j = 0; j < K; ++j)
@@ -503,9 +525,9 @@ namespace mpdg
           // domain faces).
           auto write_out = [&](auto flagged) {
               constexpr bool CM    = decltype(flagged)::value;
-              const int      cbase = wbase + K * lane + br.sz * (K * lz);
+              const int      cbase = wbase + K * lx + br.sz * (K * lz);
               T             *d0    = out + cbase;
-              const bool     x_low = lane == 0;
+              const bool     x_low = lx == 0;
               auto store = [&](int i, int j, int l) {
                 const int off = j * br.sy + l * br.sz + i;
                 const T   v   = u[(l * N + j) * N + i];
@@ -535,7 +557,7 @@ namespace mpdg
 #pragma unroll
                 for (int j = 0; j < K; ++j)
                   {
-                    if ((j == 0 && warp == 0) || (l == 0 && lz == 0))
+                    if ((j == 0 && row == 0) || (l == 0 && lz == 0))
                       {
                         if (!((j == 0 && cJ0) || (l == 0 && cL0)))
 #pragma unroll
@@ -557,16 +579,16 @@ namespace mpdg
                 for (int l = 0; l < K; ++l)
 #pragma unroll
                   for (int j = 0; j < K; ++j)
-                    if (!((j == 0 && warp == 0) || (l == 0 && lz == 0)))
+                    if (!((j == 0 && row == 0) || (l == 0 && lz == 0)))
                       add(0, j, l);
-              if (last_lane && !cIK)
+              if (x_last && !cIK)
 #pragma unroll
                 for (int l = 0; l < N; ++l)
 #pragma unroll
                   for (int j = 0; j < N; ++j)
                     if (!((j == 0 && cJ0) || (j == K && cJK) || (l == 0 && cL0) || (l == K && cLK)))
                       add(K, j, l);
-              if (last_warp && !cJK)
+              if (y_last && !cJK)
 #pragma unroll
                 for (int l = 0; l < N; ++l)
                   if (!((l == 0 && cL0) || (l == K && cLK)))
@@ -603,7 +625,7 @@ namespace mpdg
               bool con = (l == 0 && cL0) || (l == K && cLK) || (j == 0 && cJ0) || (j == K && cJK) || (i == 0 && cI0) ||
                          (i == K && cIK);
               if constexpr (MASKABLE)
-                con = con || (g.cmask != nullptr && g.cmask[wbase + K * lane + i + j * br.sy + br.sz * (K * lz + l)]);
+                con = con || (g.cmask != nullptr && g.cmask[wbase + K * lx + i + j * br.sy + br.sz * (K * lz + l)]);
               return con;
             };
             const bool masked = do_mask || (MASKABLE && mask_src && g.cmask != nullptr); // the same for the whole CTA
@@ -650,7 +672,7 @@ namespace mpdg
             if constexpr (MASKABLE)
               if (g.cmask != nullptr && mask_src && vxy)
                 {
-                  const uint8_t *cm = g.cmask + (wbase + K * lane + br.sz * (K * lz));
+                  const uint8_t *cm = g.cmask + (wbase + K * lx + br.sz * (K * lz));
 #pragma unroll
                   for (int l = 0; l < N; ++l)
 #pragma unroll

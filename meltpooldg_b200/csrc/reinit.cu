@@ -643,7 +643,7 @@ namespace mpdg
       static constexpr int value = MPDG_REINIT_MINB ? MPDG_REINIT_MINB : K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? (HEAVY ? 2 : 3) : 4) : 2);
     };
 
-    template <int K, typename T, OutMode MODE, class Op>
+    template <int K, typename T, OutMode MODE, class Op, int BX>
     __global__ void __launch_bounds__(MARCH_NT, PointMinBlocks<K, T, Op::HEAVY>::value)
     reinit_march_kernel(const __grid_constant__ typename Op::Args a)
     {
@@ -654,22 +654,32 @@ namespace mpdg
       T                                         *dst = a.dst;
       if constexpr (Op::SPLIT)
         dst = a.out[blockIdx.y];
-      march_body<K, T, MODE, Op, false, true>(a.g, a.s, a.src, dst, a.b, a.mask_src != 0, op,
+      march_body<K, T, MODE, Op, false, true, BX>(a.g, a.s, a.src, dst, a.b, a.mask_src != 0, op,
                                               reinterpret_cast<T *>(smem_raw), &s_ticket, s_bars);
+    }
+
+    template <int K, typename T, OutMode MODE, class Op, int BX>
+    cudaError_t
+    launch_point_columns(typename Op::Args &a, cudaStream_t s)
+    {
+      auto                                   kern = reinit_march_kernel<K, T, MODE, Op, BX>;
+      static std::atomic<unsigned long long> devices{0};
+      constexpr size_t                       bytes = MarchLayout<K, T, BX>::bytes;
+      if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
+        return e;
+      const unsigned ctas = march_grid(a.g, BX, MarchShape<K, T>::BZ, PointMinBlocks<K, T, Op::HEAVY>::value);
+      kern<<<dim3(ctas, Op::SPLIT ? 3 : 1), MARCH_NT, bytes, s>>>(a);
+      return cudaGetLastError();
     }
 
     template <int K, typename T, OutMode MODE, class Op>
     cudaError_t
     launch_point_kernel(typename Op::Args &a, cudaStream_t s)
     {
-      auto                                   kern = reinit_march_kernel<K, T, MODE, Op>;
-      static std::atomic<unsigned long long> devices{0};
-      constexpr size_t                       bytes = MarchLayout<K, T>::bytes;
-      if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
-        return e;
-      const unsigned ctas = march_grid(a.g, MarchShape<K, T>::BZ, PointMinBlocks<K, T, Op::HEAVY>::value);
-      kern<<<dim3(ctas, Op::SPLIT ? 3 : 1), MARCH_NT, bytes, s>>>(a);
-      return cudaGetLastError();
+      if constexpr (MODE != OutMode::BPlus) // b + A x is formed once a solve: one width
+        if (march_bx(a.g.m) != MARCH_BX)
+          return launch_point_columns<K, T, MODE, Op, MARCH_BX_NARROW>(a, s);
+      return launch_point_columns<K, T, MODE, Op, MARCH_BX>(a, s);
     }
 
     // the tangent (mode 0), the banded isotropic form (mode 0 without a normal field) or the rhs (mode 1)
@@ -865,7 +875,7 @@ namespace mpdg
   static long long
   launch_bricks(const int m[3], bool banded)
   {
-    return march_bricks(m, MarchShape<K, double>::BZ,
+    return march_bricks(m, march_bx(m), MarchShape<K, double>::BZ,
                         banded ? PointMinBlocks<K, double, BandCellOp<K, double>::HEAVY>::value :
                                  PointMinBlocks<K, double, ReinitCellOp<K, double, false>::HEAVY>::value);
   }
