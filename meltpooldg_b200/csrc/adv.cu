@@ -25,8 +25,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
-#include <set>
 
 #include "brick.cuh"
 #include "gausspoint.cuh"
@@ -336,9 +334,6 @@ namespace mpdg
     }
   };
 
-#ifndef MPDG_ADV_MINB
-#define MPDG_ADV_MINB 0
-#endif
   // CTAs (of 128 threads) per SM the register allocation is held to; measured on 80^3 FE_Q(2) FP64: affine 67 us
   // at 3, 73 at 4; SUPG 138 at 2, 186 at 3; SUPG with a field 291 at 2, 345 at 3; FP32 affine 49 at 5; 128^3
   // FE_Q(1) FP64 affine 77 at 5
@@ -346,8 +341,7 @@ namespace mpdg
   struct AdvMinBlocks
   {
     static constexpr bool f64 = sizeof(T) == 8;
-    static constexpr int  value = MPDG_ADV_MINB ? MPDG_ADV_MINB :
-                                 K == 1 ? (SUPG ? (f64 ? 3 : 5) : 5) :
+    static constexpr int  value = K == 1 ? (SUPG ? (f64 ? 3 : 5) : 5) :
                                  K == 2 ? (SUPG && VDOF ? 2 : SUPG ? (f64 ? 2 : 4) : VDOF ? (f64 ? 2 : 3) : (f64 ? 3 : 5)) : 2;
   };
 

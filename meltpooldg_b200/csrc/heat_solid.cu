@@ -201,7 +201,7 @@ namespace mpdg
     struct SolidCellOp
     {
       static constexpr int  N = K + 1, N2 = N * N, N3 = N * N * N;
-      static constexpr bool NODES = true;
+      static constexpr bool NODES = true, TANGENT = !RHS;
       const SolidArgs<T, N> &a;
       __device__ __forceinline__ SolidCell
       load(bool, int cx, int cy, int cz) const
@@ -295,7 +295,7 @@ namespace mpdg
     struct SolidDiagCellOp
     {
       static constexpr int  N = K + 1, N2 = N * N, N3 = N * N * N;
-      static constexpr bool NODES = true;
+      static constexpr bool NODES = true, TANGENT = false;
       const SolidArgs<T, N> &a;
       __device__ __forceinline__ SolidCell
       load(bool, int cx, int cy, int cz) const
@@ -351,19 +351,17 @@ namespace mpdg
       }
     };
 
-#ifndef MPDG_SOLID_MINB
-#define MPDG_SOLID_MINB 0
-#endif
-    // CTAs (of 128 threads) per SM the register allocation is held to; residual, diagonal and tangent, 64^3 FE_Q(2) FP64:
-    // 490 us at 3, 576 at 2, 590 at 4 (1007 before)
-    template <int K, typename T>
+    // CTAs (of 128 threads) per SM the register allocation is held to.  FE_Q(2) FP64 at 2 and 3: tangent 72^3 273 and
+    // 318 us, 80x64x48 206 and 209, 33x33x40 77 and 75 (1.2 KB of spills per thread at 3); residual 80x64x48 176
+    // and 171, diagonal 201 and 197
+    template <int K, typename T, bool TANGENT>
     struct SolidMinBlocks
     {
-      static constexpr int value = MPDG_SOLID_MINB ? MPDG_SOLID_MINB : K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? 3 : 4) : 2);
+      static constexpr int value = K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? (TANGENT ? 2 : 3) : 4) : 2);
     };
 
     template <int K, typename T, OutMode MODE, class Op, int BX>
-    __global__ void __launch_bounds__(MARCH_NT, SolidMinBlocks<K, T>::value)
+    __global__ void __launch_bounds__(MARCH_NT, SolidMinBlocks<K, T, Op::TANGENT>::value)
     heat_solid_kernel(const __grid_constant__ SolidArgs<T, K + 1> a)
     {
       extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -412,7 +410,7 @@ namespace mpdg
       constexpr size_t                       bytes = MarchLayout<K, T, BX>::bytes;
       if (cudaError_t e = ensure_smem(kern, bytes, devices); e != cudaSuccess)
         return e;
-      const unsigned ctas = march_grid(a.g, BX, MarchShape<K, T>::BZ, SolidMinBlocks<K, T>::value);
+      const unsigned ctas = march_grid(a.g, BX, MarchShape<K, T>::BZ, SolidMinBlocks<K, T, Op::TANGENT>::value);
       kern<<<ctas, MARCH_NT, bytes, stream>>>(a);
       return cudaGetLastError();
     }
@@ -505,9 +503,9 @@ namespace mpdg
   long long
   heat_solid_launch_bricks(int K, const int m[3])
   {
-    return K == 1 ? march_bricks(m, march_bx(m), MarchShape<1, double>::BZ, SolidMinBlocks<1, double>::value) :
-                    (K == 2 ? march_bricks(m, march_bx(m), MarchShape<2, double>::BZ, SolidMinBlocks<2, double>::value) :
-                              march_bricks(m, march_bx(m), MarchShape<3, double>::BZ, SolidMinBlocks<3, double>::value));
+    return K == 1 ? march_bricks(m, march_bx(m), MarchShape<1, double>::BZ, SolidMinBlocks<1, double, true>::value) :
+                    (K == 2 ? march_bricks(m, march_bx(m), MarchShape<2, double>::BZ, SolidMinBlocks<2, double, true>::value) :
+                              march_bricks(m, march_bx(m), MarchShape<3, double>::BZ, SolidMinBlocks<3, double, true>::value));
   }
 
   template <typename T>

@@ -20,7 +20,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "brick.cuh"
 #include "gausspoint.cuh"
@@ -632,15 +631,12 @@ namespace mpdg
       }
     };
 
-#ifndef MPDG_REINIT_MINB
-#define MPDG_REINIT_MINB 0
-#endif
     // CTAs (of 128 threads) per SM the register allocation is held to; tangent and rhs, 72x56x64 FE_Q(2) FP64: 288 us at
     // 2 (1250 before, point by point over the nodes), 343 at 3; normal, curvature and banded apply 310 at 3, 348 at 4
     template <int K, typename T, bool HEAVY>
     struct PointMinBlocks
     {
-      static constexpr int value = MPDG_REINIT_MINB ? MPDG_REINIT_MINB : K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? (HEAVY ? 2 : 3) : 4) : 2);
+      static constexpr int value = K == 1 ? 6 : (K == 2 ? (sizeof(T) == 8 ? (HEAVY ? 2 : 3) : 4) : 2);
     };
 
     template <int K, typename T, OutMode MODE, class Op, int BX>
