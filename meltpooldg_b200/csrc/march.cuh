@@ -110,13 +110,15 @@ namespace mpdg
     return (unsigned)g.nbr[0] * g.nbr[1] * g.nbr[2];
   }
 
+  // CTAs that a launch has at least, in columns of width bx or (its b + A x form) MARCH_BX
   inline long long
   march_bricks(const int m[3], int bx, int bz_full, int per_sm)
   {
     GridDesc g{};
     for (int d = 0; d < 3; ++d)
       g.m[d] = m[d];
-    return march_grid(g, bx, bz_full, per_sm);
+    const unsigned n = march_grid(g, bx, bz_full, per_sm), wide = march_grid(g, MARCH_BX, bz_full, per_sm);
+    return n < wide ? n : wide;
   }
 
   // flags / dot partials an operator must hold for the segments of any of its marching applies
