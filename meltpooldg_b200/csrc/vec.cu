@@ -1,9 +1,9 @@
 // Vector kernels and deterministic reductions for the Krylov solvers.
 //
-// Every reduction runs on a fixed grid of RED_BLOCKS blocks with a grid-stride loop, reduces in
-// registers/shared memory in a fixed order, writes one partial per block, and the last block to
-// finish (threadfence + ticket) sums the partials in block order.  Results are therefore
-// bit-reproducible run to run.  Sums are accumulated in double for every vector type, so the FP32
+// Every reduction runs on a fixed grid (RED_BLOCKS blocks; the Gram-Schmidt kernels at most as many, all
+// resident) with a grid-stride loop, reduces in registers/shared memory in a fixed order, writes one
+// partial per block, and the last block to finish (threadfence + ticket) sums the partials in a fixed
+// order.  Results are therefore bit-reproducible run to run.  Sums are accumulated in double for every vector type, so the FP32
 // inner solver keeps FP64 dot products and norms.
 //
 // The PCG kernels carry the scalar recurrences of dealii::SolverCG on the device (CGState): the
@@ -80,19 +80,40 @@ namespace mpdg
       __syncthreads();
       if (!last)
         return;
-      // one warp per value: up to 33 values (GMRES) without a barrier between them
-      for (int k = warp; k < m_active; k += NWARP)
+      auto sum = [&](int k, int first, int step) { // of value k over the blocks first, first + step, ..., by a warp
+        double s = MAX ? -INFINITY : 0.0;
+        for (int b = first + lane; b < (int)gridDim.x; b += step)
+          {
+            const double p = __ldcg(red.partials + k * RED_BLOCKS + b);
+            s              = MAX ? fmax(s, p) : s + p;
+          }
+        return MAX ? warp_max(s) : warp_sum(s);
+      };
+      if constexpr (M <= 2)
         {
-          double s = MAX ? -INFINITY : 0.0;
-          for (int b = lane; b < (int)gridDim.x; b += 32)
-            {
-              const double p = __ldcg(red.partials + k * RED_BLOCKS + b);
-              s              = MAX ? fmax(s, p) : s + p;
-            }
-          s = MAX ? warp_max(s) : warp_sum(s);
+          // CG's one or two values by all warps: the loads of a value are a chain at the end of every iteration
+          // (three-pass CG, FE_Q(4) 24^3: 41.2 us an iteration, 43.2 by one warp per value)
+          constexpr int PER = NWARP / M;
+          const double  s   = sum(warp / PER, 32 * (warp % PER), 32 * PER);
           if (lane == 0)
-            tot[k] = s;
+            sh[warp / PER][warp % PER] = s;
+          __syncthreads();
+          if (threadIdx.x < M)
+            {
+              double t = sh[threadIdx.x][0];
+              for (int w = 1; w < PER; ++w)
+                t = MAX ? fmax(t, sh[threadIdx.x][w]) : t + sh[threadIdx.x][w];
+              tot[threadIdx.x] = t;
+            }
         }
+      else
+        // one warp per value: up to 33 values (GMRES) without a barrier between them
+        for (int k = warp; k < m_active; k += NWARP)
+          {
+            const double s = sum(k, 0, 32);
+            if (lane == 0)
+              tot[k] = s;
+          }
       __syncthreads();
       if (threadIdx.x == 0)
         {
