@@ -470,7 +470,9 @@ namespace mpdg
 #define MPDG_MARCH_MINB1_F32 10
 #endif
   // CTAs per SM the register allocation of the column-marching kernel is held to (FE_Q(2) FP64 96^3: 60.2 us
-  // at 4, 63.2 at 5, 67.3 at 6; FP32 131x97x118: 84.3 at 7, 87.8 at 8; FE_Q(1) FP64 192^3: 142 at 10, 147 at 8)
+  // at 4, 63.2 at 5, 67.3 at 6; FP32 131x97x118: 84.3 at 7, 87.8 at 8; FE_Q(1) FP64 192^3: 142 at 10, 147 at 8).
+  // With the fused dot the difference is within 1.5 % either way: three-pass CG at 4 and 5, 96^3 178.0 and 179.2 us
+  // an iteration, 128^3 408 and 406; mixed with it, FP32 at 7 and 8, 96^3 9.37 and 9.24 ms, 128^3 25.8 and 26.1
   template <int K, typename T>
   struct MarchMinBlocks
   {

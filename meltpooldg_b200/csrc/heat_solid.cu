@@ -149,7 +149,7 @@ namespace mpdg
     {
       long long first; // the cell's first lattice point
     };
-    template <typename T, int N>
+    template <int N>
     __device__ __forceinline__ SolidCell
     solid_cell(const GridDesc &g, int cx, int cy, int cz)
     {
@@ -206,7 +206,7 @@ namespace mpdg
       __device__ __forceinline__ SolidCell
       load(bool, int cx, int cy, int cz) const
       {
-        return solid_cell<T, N>(a.g, cx, cy, cz);
+        return solid_cell<N>(a.g, cx, cy, cz);
       }
       __device__ __forceinline__ void
       apply(T *R, const MarchNodes<K, T> &nodes, const SolidCell &c) const
@@ -300,7 +300,7 @@ namespace mpdg
       __device__ __forceinline__ SolidCell
       load(bool, int cx, int cy, int cz) const
       {
-        return solid_cell<T, N>(a.g, cx, cy, cz);
+        return solid_cell<N>(a.g, cx, cy, cz);
       }
       __device__ __forceinline__ void
       apply(T *R, const MarchNodes<K, T> &, const SolidCell &c) const

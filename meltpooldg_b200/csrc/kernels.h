@@ -83,7 +83,7 @@ namespace mpdg
     const int    *skip = nullptr;
   };
 
-  // ---- temperature-dependent material (solid / liquid phases, heat_solid.cu), FE_Q(1, 2)
+  // ---- temperature-dependent material (solid / liquid phases, heat_solid.cu), FE_Q(1..3)
   struct SolidMaterial
   {
     double rho_l = 1.0, cp_l = 1.0, k_l = 1.0; // liquid
@@ -123,7 +123,7 @@ namespace mpdg
                                   const double hlen[3], const double *temp, const double *temp_old, double *diag,
                                   cudaStream_t s);
 
-  // ---- conservative level-set reinitialisation (Olsson, reinit.cu), FE_Q(1, 2)
+  // ---- conservative level-set reinitialisation (Olsson, reinit.cu), FE_Q(1..3)
   template <typename T>
   struct ReinitLaunch
   {

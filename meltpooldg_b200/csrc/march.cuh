@@ -1,18 +1,18 @@
 // Column-marching apply for low degrees: one thread per cell, no shared-memory reduction.
 //
-// A CTA of 4 warps owns a column of 32 x 4 cells (x, y) and marches through a segment of bz cell
-// layers in z.  Lane = cell x-index, warp = cell y-index.  Per layer:
+// A CTA of 4 warps owns a column of 32 x 4 cells (x, y; march_bx: or 16 x 8) and marches through a segment of
+// bz cell layers in z, a cell per thread in rows along x.  Per layer:
 //   1. the K new lattice planes of the layer arrive in a ring of 2 K + 1 planes by bulk copies
 //      (cp.async.bulk, one per lattice row, issued by the lanes of warp 0 two layers ahead); the plane
 //      shared with the layer below stays in the ring;
 //   2. each thread applies the cell operator to its cell's (K+1)^3 values in registers;
-//   3. x-neighbours combine their common face with warp shuffles (lane t adds lane t-1's x = K face
-//      into its x = 0 face), y-neighbours through a small shared exchange buffer (two buffers taken in
+//   3. x-neighbours combine their common face with warp shuffles (a cell adds its lower neighbour's x = K
+//      face into its x = 0 face), y-neighbours through a small shared exchange buffer (two buffers taken in
 //      turn: one barrier per layer), z-neighbours by carrying the z = K face in registers;
 //   4. each thread then owns the points i, j, l in [0, K) of its cell and writes them with coalesced
 //      stores; points on the faces shared with neighbouring columns / segments are combined with global
 //      atomics, initialised by their owner through the ticket / flag handshake of brick.cuh.  The
-//      column's high x face (one lane) and high y face (one warp) add straight from the cell's values,
+//      column's high x face and high y face add straight from the values of the cells there,
 //      so neither the exchange nor the carry handles them.
 //
 // Staging.  A lattice row of n points starts at any element, a bulk copy at a 16-byte boundary: the copy
@@ -70,10 +70,11 @@ namespace mpdg
   // Segment length for a mesh: the bz whose CTAs take the least time on the resident slots.  In units of
   // a layer at full occupancy a CTA costs its layers plus about one (two, where it starts on an idle
   // slot: handshake and the first planes' latency); the last wave, of which only a part of the slots is
-  // in use, takes 0.57 + 0.43 part of that per layer (FE_Q(2) FP64, 96^3: 5.6 us a layer at 4.9 CTAs
-  // per SM, 4.5 at 2.9, 3.9 at 1.5).  Measured against it, FE_Q(2) FP64: 96^3 67 us at bz = 10 (one
-  // full wave) against 88 at 8 (864 segments on 740 slots) and 81 at 16; 64^3 25 us at 3 against 36 at
-  // 8; 32^3 10 us at 1 against 33 at 8.
+  // in use, takes 0.57 + 0.43 part of that per layer (fitted to the FE_Q(2) FP64 heat apply at five CTAs per
+  // SM: 5.6 us a layer at 4.9 CTAs per SM, 4.5 at 2.9, 3.9 at 1.5).  What it picks, and its neighbours, heat
+  // apply: FE_Q(2) FP64 (592 slots) 96^3 58.0 us at bz = 12 (one wave of 576), 68 at 8, 64 at 16, 80 at 24;
+  // 64^3 24.7 at 4, 27.7 at 2, 31.0 at 8; 32^3 10.6 at 1, 16.8 at 4; FP32 128^3 91.7 at 16, 93.7 at 8, 103 at
+  // 12; FE_Q(1) FP64 192^3 143 us, 149 to 153 at 8 to 24.  The other operators take the same rule.
   inline int
   march_plan(const int m[3], int bx, int bz_full, int slots, int *nseg)
   {

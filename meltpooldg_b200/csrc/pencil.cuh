@@ -83,9 +83,10 @@ namespace mpdg
 
   // Parts of z for a mesh: the number of nearly equal parts whose bricks take the least time on the
   // resident slots (the cost model of march_plan), or the full-height bricks where that gains less than
-  // 15 % by the model.  Measured at 64^3: FE_Q(3) FP64 16 parts 78.8 us (1024 bricks on 740 slots), 11 parts
-  // one wave, 72 us; FE_Q(4) FP64 16 parts 120.6, 9 parts (one wave, 12 % by the model) 121.8.  Small meshes
-  // gain the most: full-height bricks leave most slots without one.
+  // 15 % by the model.  Measured at 64^3: FE_Q(3) FP64 16 parts 83.2 us (1024 bricks on 740 slots), 11 parts
+  // (one wave) 69.3; FE_Q(4) FP64 16 parts 120.3, 9 parts (one wave, 12 % by the model) 120.5.  The model was
+  // fitted to the marching apply and is an estimate here: it misses FE_Q(4) FP32 64^3, 90.3 us at 9 parts and 97.2
+  // at 16.  Small meshes gain the most: full-height bricks leave most slots without one.
   inline int
   pencil_plan(const int m[3], int bx, int by, int bz_full, int slots)
   {

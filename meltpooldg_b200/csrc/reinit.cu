@@ -54,7 +54,6 @@ namespace mpdg
     {
       int c[3];
     };
-    template <typename T, int N>
     __device__ __forceinline__ PointCell
     point_cell(const GridDesc &g, int cx, int cy, int cz)
     {
@@ -374,7 +373,7 @@ namespace mpdg
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
-        return point_cell<T, N>(a.g, cx, cy, cz);
+        return point_cell(a.g, cx, cy, cz);
       }
       __device__ __forceinline__ void
       apply(T *R, const MarchNodes<K, T> &nodes, const PointCell &c) const
@@ -435,7 +434,7 @@ namespace mpdg
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
-        return point_cell<T, N>(a.g, cx, cy, cz);
+        return point_cell(a.g, cx, cy, cz);
       }
       template <bool DOT>
       __device__ __forceinline__ double
@@ -489,7 +488,7 @@ namespace mpdg
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
-        return point_cell<double, N>(a.g, cx, cy, cz);
+        return point_cell(a.g, cx, cy, cz);
       }
       __device__ __forceinline__ double *
       out(int m) const
@@ -580,7 +579,7 @@ namespace mpdg
       __device__ __forceinline__ PointCell
       load(bool, int cx, int cy, int cz) const
       {
-        return point_cell<double, N>(a.g, cx, cy, cz);
+        return point_cell(a.g, cx, cy, cz);
       }
       template <bool DOT>
       __device__ __forceinline__ double
