@@ -12,7 +12,7 @@
 // Differences of values that were interpolated before carry that interpolation's rounding, amplified by
 // |u| / (h |grad u|).  So a gradient alone differences the nodal values and interpolates the differences
 // (gp_gradient), and an operator that takes values and gradient from one interpolation subtracts the cell's
-// middle node first.  The tables are products formed in extended precision and rounded once.  Against 80-bit
+// middle node first; their tables are products formed in extended precision and rounded once.  Against 80-bit
 // values, FE_Q(2) 35x22x27: right-hand side of the reinitialisation 4.9e-14 without the three, 2.9e-15 with them
 // (plain sums over the 27 nodes: 1.8e-14), normal 2.8e-15 and 2.5e-16 (1.1e-15), at the same time per apply.
 #pragma once
@@ -48,27 +48,26 @@ namespace mpdg
     T G[3][N * (N - 1)]; // derivative of the nodal values at the points, 1 / h_d G, on differences
     T Gzt[N * N];        // weighted transpose of the z derivative (rows: nodes), with the volume
 
-    // every entry is computed in extended precision and rounded once
+    // from B, G, Dq and qw of Tables1D, entries computed in R and rounded (from long double: once)
+    template <typename R>
     void
-    fill(const Tables1D &t, const double h[3])
+    fill(const R *tB, const R *tG, const R *tD, const R *tw, const double h[3])
     {
-      using real = long double;
       for (int q = 0; q < N; ++q)
         for (int r = 0; r < N; ++r)
           {
-            const real b = t.ext.B[q * N + r], w = t.ext.qw[q];
-            B[q * N + r]   = (T)b;
-            Gzt[r * N + q] = (T)((real)h[0] * h[1] * w * t.ext.G[q * N + r]);
+            B[q * N + r]   = (T)tB[q * N + r];
+            Gzt[r * N + q] = (T)((R)h[0] * h[1] * tw[q] * tG[q * N + r]);
             for (int d = 0; d < 3; ++d)
               {
-                Bt[d][r * N + q] = (T)((d == 2 ? (real)h[0] * h[1] * h[2] : real(1)) * w * b);
-                P[d][q * N + r]  = (T)(t.ext.Dq[r * N + q] * t.ext.qw[r] / w / h[d]);
+                Bt[d][r * N + q] = (T)((d == 2 ? (R)h[0] * h[1] * h[2] : R(1)) * tw[q] * tB[q * N + r]);
+                P[d][q * N + r]  = (T)(tD[r * N + q] * tw[r] / tw[q] / h[d]);
               }
           }
       for (int d = 0; d < 3; ++d)
         {
-          gp_on_differences<T, N>(t.ext.Dq, real(1) / h[d], D[d]);
-          gp_on_differences<T, N>(t.ext.G, real(1) / h[d], G[d]);
+          gp_on_differences<T, N>(tD, R(1) / h[d], D[d]);
+          gp_on_differences<T, N>(tG, R(1) / h[d], G[d]);
         }
     }
   };

@@ -434,7 +434,9 @@ namespace mpdg
       a.g = h.grid;
       a.s = h.sync;
       a.m = solid_mat<T>(h.mat);
-      a.t.fill(tables(K), h.hlen);
+      // tables from doubles, as the diagonal's: the gradient of a temperature of 1e3 K rounds far above them
+      const Tables1D &t = tables(K);
+      a.t.fill(t.B, t.G, t.Dq, t.qw, h.hlen);
       const double scale = h.rhs ? -1.0 : h.scale;
       for (int i = 0; i < N * N; ++i)
         {
@@ -479,7 +481,7 @@ namespace mpdg
       a.g = g;
       a.s = sync;
       a.m = solid_mat<double>(mat);
-      a.t.fill(t, hlen);
+      a.t.fill(t.B, t.G, t.Dq, t.qw, hlen);
       a.inv_dt = 1.0 / dt;
       for (int d = 0; d < 3; ++d)
         for (int q = 0; q < N; ++q)

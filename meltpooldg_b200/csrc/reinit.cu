@@ -688,7 +688,7 @@ namespace mpdg
       const bool          banded = h.band > 0.0 && h.band_ls != nullptr;
       a.g                        = h.grid;
       a.s                        = h.sync;
-      a.t.fill(t, h.hlen);
+      a.t.fill(t.ext.B, t.ext.G, t.ext.Dq, t.ext.qw, h.hlen);
       if (h.normal[0] == nullptr) // the banded form's flux: D carries the diffusivity
         for (int d = 0; d < 3; ++d)
           gp_on_differences<T, N>(t.ext.Dq, (long double)h.scale * h.eps_tangential / h.hlen[d], a.t.D[d]);
@@ -818,7 +818,8 @@ namespace mpdg
       GradientArgs<K> a{};
       a.g = g;
       a.s = sync;
-      a.t.fill(tables(K), hlen);
+      const Tables1D &t = tables(K);
+      a.t.fill(t.ext.B, t.ext.G, t.ext.Dq, t.ext.qw, hlen);
       a.src      = in[0];
       a.mask_src = 0;
       a.band_ls  = band > 0.0 ? band_ls : nullptr;
